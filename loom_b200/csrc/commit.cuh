@@ -246,7 +246,7 @@ inline void launch_leaves(Ctx& c, const std::vector<LeafGroup>& gs) {
   uint64_t all_leaves = 0;
   for (auto& g : gs) all_leaves += g.n_leaves;
   bool per_thread = p2_per_thread(c, all_leaves, c.tune.p2_leaf_min_per_sm);
-  const unsigned lb = c.tune.leaf_block;
+  const unsigned lb = std::min<unsigned>(c.tune.leaf_block, P2_MAX_BLOCK);
   c.timed("hash_leaves", bytes, perms, [&] {
     if (per_thread)
       k_hash_leaves1<<<dim3((max_leaves + lb - 1) / lb, (unsigned)gs.size()), lb, 0, c.stream>>>((const LeafGroup*)tab->p);
@@ -343,7 +343,7 @@ inline bool build_tree(Ctx& c, TreeDev& t, bool read_root = true, const FsTail* 
       if (p2_per_thread(c, start, c.tune.p2_inject_min_per_sm)) {
         // small blocks (one warp by default): chains are few (down to ~200
         // per SM) and long, so small blocks spread them evenly over the SMs
-        const unsigned ib = c.tune.inject_block;
+        const unsigned ib = std::min<unsigned>(c.tune.inject_block, P2_MAX_BLOCK);
         k_merkle_inject1<<<(start + ib - 1) / ib, ib, 0, c.stream>>>(t.nodes->p, start, tab, cnt);
       } else
         k_merkle_inject<<<(start + 19) / 20, 128, 0, c.stream>>>(t.nodes->p, start, tab, cnt);
@@ -373,7 +373,7 @@ inline bool build_tree(Ctx& c, TreeDev& t, bool read_root = true, const FsTail* 
     c.timed(blocks == 1 ? "merkle_tail" : "merkle_level", 96.0 * perms, perms, [&] {
       // at least one warp: the challenge needs one
       const unsigned thr = std::max(32u, tail_threads(top / blocks, fold_first));
-      k_merkle_tail<<<blocks, thr, 0, c.stream>>>(t.nodes->p, top, fold_first, (const InjRef*)ref_tab->p,
+      k_merkle_tail<<<blocks, thr, p2c_smem_words(thr / 32) * 4, c.stream>>>(t.nodes->p, top, fold_first, (const InjRef*)ref_tab->p,
                                                   (uint32_t)refs.size(), with_fs ? *fs : FsTail{});
       LG_LAUNCH();
     });

@@ -353,9 +353,15 @@ __device__ __forceinline__ uint32_t leaf_elem(const LeafGroup& g, uint32_t idx, 
   return g.ext[e * g.stride + 2 * k + h];
 }
 
+// Kernels with a permutation per thread: built for blocks of at most 256
+// threads and 128 registers, since the permutation keeps its 24 words and the
+// products in flight in registers.  With a cap of 64 registers (1024-thread
+// blocks) the full rounds take 6.9 SM clocks instead of 6.4 (B200).
+constexpr int P2_MAX_BLOCK = 256;
+
 // One thread per leaf: the fewest instructions per permutation, for launches
 // with enough leaves to fill the GPU.
-__global__ void k_hash_leaves1(const LeafGroup* groups) {
+__global__ void __launch_bounds__(P2_MAX_BLOCK, 2) k_hash_leaves1(const LeafGroup* groups) {
   const LeafGroup g = groups[blockIdx.y];
   uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= g.n_leaves) return;
@@ -379,7 +385,7 @@ __global__ void k_hash_leaves1(const LeafGroup* groups) {
 constexpr uint32_t P2_GROUPS_PER_WARP = 5;
 
 __global__ void k_hash_leaves(const LeafGroup* groups) {
-  __shared__ uint32_t keys[144];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
   L.init();
@@ -430,7 +436,7 @@ __device__ __forceinline__ void p2c_store_digest(const uint32_t x[4], const P2La
   }
 }
 
-__device__ __forceinline__ void merkle_node(uint32_t* nodes, uint64_t id, const P2Lane& L, const uint32_t* keys,
+__device__ __forceinline__ void merkle_node(uint32_t* nodes, uint64_t id, const P2Lane& L, uint32_t* keys,
                                             bool active) {
   uint32_t x[4] = {0, 0, 0, 0};
   p2c_load_slot(x, L, 1, nodes + 2 * id * 8, active);
@@ -441,7 +447,7 @@ __device__ __forceinline__ void merkle_node(uint32_t* nodes, uint64_t id, const 
 
 // node = H(... H(H(node, inj_0[j]), inj_1[j]) ..., inj_{n-1}[j])
 __device__ __forceinline__ void merkle_chain(uint32_t* nodes, uint64_t id, uint32_t j, const uint32_t* const* inj,
-                                             uint32_t n_inj, const P2Lane& L, const uint32_t* keys, bool active) {
+                                             uint32_t n_inj, const P2Lane& L, uint32_t* keys, bool active) {
   if (n_inj == 0) return;
   uint32_t x[4] = {0, 0, 0, 0};
   p2c_load_slot(x, L, 1, nodes + id * 8, active);
@@ -454,7 +460,7 @@ __device__ __forceinline__ void merkle_chain(uint32_t* nodes, uint64_t id, uint3
 }
 
 __global__ void k_merkle_level(uint32_t* nodes, uint32_t start) {
-  __shared__ uint32_t keys[144];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
   L.init();
@@ -464,7 +470,7 @@ __global__ void k_merkle_level(uint32_t* nodes, uint32_t start) {
 }
 
 __global__ void k_merkle_inject(uint32_t* nodes, uint32_t start, const uint32_t* const* inj, uint32_t n_inj) {
-  __shared__ uint32_t keys[144];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
   L.init();
@@ -484,7 +490,7 @@ __device__ __forceinline__ void st_digest(uint32_t* p, const uint32_t d[8]) {
   reinterpret_cast<uint4*>(p)[0] = make_uint4(d[0], d[1], d[2], d[3]);
   reinterpret_cast<uint4*>(p)[1] = make_uint4(d[4], d[5], d[6], d[7]);
 }
-__global__ void k_merkle_level1(uint32_t* nodes, uint32_t start) {
+__global__ void __launch_bounds__(P2_MAX_BLOCK, 2) k_merkle_level1(uint32_t* nodes, uint32_t start) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= start) return;
   const uint64_t id = (uint64_t)start + i;
@@ -494,7 +500,7 @@ __global__ void k_merkle_level1(uint32_t* nodes, uint32_t start) {
   p2_compress(to_mont(NODE_TAG), l, r, l);
   st_digest(nodes + id * 8, l);
 }
-__global__ void k_merkle_inject1(uint32_t* nodes, uint32_t start, const uint32_t* const* inj, uint32_t n_inj) {
+__global__ void __launch_bounds__(P2_MAX_BLOCK, 2) k_merkle_inject1(uint32_t* nodes, uint32_t start, const uint32_t* const* inj, uint32_t n_inj) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= start) return;
   uint32_t* nd = nodes + ((uint64_t)start + j) * 8;
@@ -522,7 +528,7 @@ struct InjRef { const uint32_t* leaves; uint32_t width; };
 struct FsTail { const uint32_t* pre; uint32_t n_pre; const uint32_t* prev; uint32_t* out; };
 __global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, const InjRef* inj, uint32_t n_inj,
                               FsTail fs) {
-  __shared__ uint32_t keys[144];
+  extern __shared__ __align__(16) uint32_t keys[];  // p2c_smem_words(warps)
   __shared__ const uint32_t* chain[64];
   __shared__ uint32_t msg[64];
   p2_load_full_keys(keys);
@@ -578,7 +584,7 @@ __global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, con
 
 // Permutation test hook: one state of 24 words per group of six lanes.
 __global__ void k_p2_permute(uint32_t* states, uint64_t n) {
-  __shared__ uint32_t keys[144];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
   L.init();
@@ -1250,7 +1256,7 @@ struct FriRound {
 __global__ void __launch_bounds__(1024) k_fri_tail(const FriRound* rounds, uint32_t n_rounds, uint32_t j0,
                                                    const AxpyTerm* terms, const uint32_t* pre, uint32_t* chal,
                                                    uint32_t inv2) {
-  __shared__ uint32_t keys[144];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(32)];
   __shared__ uint32_t msg[64];
   p2_load_full_keys(keys);  // ends with a barrier
   P2Lane L;
@@ -1355,7 +1361,7 @@ __global__ void __launch_bounds__(1024) k_fri_tail(const FriRound* rounds, uint3
 // per permutation; `out` gets 8 words.
 __global__ void k_fs_challenge(const uint32_t* pre, uint32_t n_pre, const uint32_t* prev, const uint32_t* bind,
                                uint32_t* out) {
-  __shared__ uint32_t keys[144];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(1)];
   __shared__ uint32_t msg[64];
   const uint32_t total = n_pre + 16;  // n_pre <= 48, checked by the host
   for (uint32_t i = threadIdx.x; i < total; i += blockDim.x)
@@ -1392,7 +1398,7 @@ struct FsSeg { const uint32_t* src; uint32_t len, off; };
 struct FsChal { uint32_t moff, total; uint32_t* out; int32_t fwd; };
 __global__ void __launch_bounds__(32) k_fs_chain(const FsChal* chals, uint32_t n_chals, const FsSeg* segs,
                                                  uint32_t n_segs) {
-  __shared__ uint32_t keys[144];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(1)];
   __shared__ uint32_t msg[FS_MAX_MSG];
   for (uint32_t s = threadIdx.x; s < n_segs; s += blockDim.x) {
     const FsSeg sg = segs[s];

@@ -74,15 +74,8 @@ LG_HD void p2_internal(uint32_t s[24]) {
 
 LG_HD uint32_t p2_cube(uint32_t x) { return mul(mul_lazy(x, x), x); }
 
-// Unrolling of the round loops.  A fully unrolled permutation is ~9K
-// instructions, more than the SM's instruction caches hold when warps drift
-// apart; rolled round loops keep the hot code small.
-#ifndef LG_P2_FULL_UNROLL
-#define LG_P2_FULL_UNROLL 1
-#endif
-#ifndef LG_P2_PARTIAL_UNROLL
-#define LG_P2_PARTIAL_UNROLL 3
-#endif
+// The round loops stay rolled: a fully unrolled permutation is more code than
+// the SM's instruction caches hold when warps drift apart.
 #define LG_PRAGMA(x) _Pragma(#x)
 #define LG_UNROLL(n) LG_PRAGMA(unroll n)
 
@@ -96,19 +89,6 @@ LG_HD void p2_full_round(uint32_t s[24], const uint32_t* rk) {
 template <int N> LG_HD uint32_t tree_sum(const uint32_t* v) {
   if constexpr (N == 1) return v[0];
   else return add(tree_sum<N / 2>(v), tree_sum<N - N / 2>(v + N / 2));
-}
-
-// Sum of N values in [0, p) as a 64-bit integer (two instructions a term,
-// against three for a reduced addition), reduced once: with v < 2^37,
-// v = hi 2^32 + lo = lo + hi (2^32 mod p); 2^32 mod p is MONT_ONE.
-template <int N> LG_HD uint32_t wide_sum(const uint32_t* v) {
-  static_assert(N <= 32, "the sum must stay below 2^37");
-  uint64_t acc = 0;
-#pragma unroll
-  for (int i = 0; i < N; i++) acc += v[i];
-  const uint64_t t = (uint64_t)(uint32_t)(acc >> 32) * MONT_ONE + (uint32_t)acc;  // < 2^32 + 2^30
-  const uint32_t r = (uint32_t)t + (uint32_t)(t >> 32) * MONT_ONE;               // < 2^32
-  return red(red(r));                                                            // [0, 2^32) -> [0, p)
 }
 
 constexpr uint32_t P2_DIAG_C[24] = LG_P2_DIAG_INIT;
@@ -136,9 +116,9 @@ __constant__ P2DiagShoup P2_DSH_D = make_p2_diag_shoup();
 #else
 #define LG_P2_DSH P2_DSH_H
 #endif
-constexpr uint32_t C23 = 23, C23_SH = shoup(23);
+constexpr uint32_t C23 = 23, C23_SH = shoup(23);  // the carried sum (p2_coop.cuh)
 
-// Products by the diagonal entries +-2^-k (17 of the 24).  With
+// Products by +-2^-k (17 of the 24 diagonal entries, and squares of them).  With
 // x = hi 2^k + lo (lo < 2^k) and 2^k (p - 1)/2^k = p - 1 = -1 mod p,
 //   x 2^-k = hi + lo 2^-k = hi - lo (p - 1)/2^k  (mod p):
 // a shift, a mask and one multiply by a small constant in place of Shoup's
@@ -156,88 +136,148 @@ constexpr uint32_t cx_pow2_inv(int k, bool neg) {
   const uint32_t v = cx_pow((P + 1) / 2, (uint64_t)k);
   return neg ? (P - v) % P : v;
 }
-#define LG_P2_DIAG_POW2(i, k, neg) \
-  static_assert(P2_DSH_H.w[i] == cx_pow2_inv(k, neg), "internal diagonal entry " #i " is " #neg " 2^-" #k)
-LG_P2_DIAG_POW2(3, 1, false);
-LG_P2_DIAG_POW2(6, 1, true);
-LG_P2_DIAG_POW2(9, 8, false);
-LG_P2_DIAG_POW2(10, 2, false);
-LG_P2_DIAG_POW2(11, 3, false);
-LG_P2_DIAG_POW2(12, 4, false);
-LG_P2_DIAG_POW2(13, 5, false);
-LG_P2_DIAG_POW2(14, 6, false);
-LG_P2_DIAG_POW2(15, 24, false);
-LG_P2_DIAG_POW2(16, 8, true);
-LG_P2_DIAG_POW2(17, 3, true);
-LG_P2_DIAG_POW2(18, 4, true);
-LG_P2_DIAG_POW2(19, 5, true);
-LG_P2_DIAG_POW2(20, 6, true);
-LG_P2_DIAG_POW2(21, 7, true);
-LG_P2_DIAG_POW2(22, 9, true);
-LG_P2_DIAG_POW2(23, 24, true);
-#undef LG_P2_DIAG_POW2
 
-// d_i s_i for i = 2..23 into p[2..23], for s_i < 2p; outputs in [0, p).
-// Entries 2, 4, 5, 7, 8 (2, 3, 4, -3, -4) use Shoup's products.
-LG_HD void p2_diag_products(const uint32_t s[24], uint32_t p[24]) {
-  p[2] = mulc(s[2], LG_P2_DSH.w[2], LG_P2_DSH.ws[2]);
-  p[3] = mul_pow2_inv<1, false>(s[3]);
-  p[4] = mulc(s[4], LG_P2_DSH.w[4], LG_P2_DSH.ws[4]);
-  p[5] = mulc(s[5], LG_P2_DSH.w[5], LG_P2_DSH.ws[5]);
-  p[6] = mul_pow2_inv<1, true>(s[6]);
-  p[7] = mulc(s[7], LG_P2_DSH.w[7], LG_P2_DSH.ws[7]);
-  p[8] = mulc(s[8], LG_P2_DSH.w[8], LG_P2_DSH.ws[8]);
-  p[9] = mul_pow2_inv<8, false>(s[9]);
-  p[10] = mul_pow2_inv<2, false>(s[10]);
-  p[11] = mul_pow2_inv<3, false>(s[11]);
-  p[12] = mul_pow2_inv<4, false>(s[12]);
-  p[13] = mul_pow2_inv<5, false>(s[13]);
-  p[14] = mul_pow2_inv<6, false>(s[14]);
-  p[15] = mul_pow2_inv<24, false>(s[15]);
-  p[16] = mul_pow2_inv<8, true>(s[16]);
-  p[17] = mul_pow2_inv<3, true>(s[17]);
-  p[18] = mul_pow2_inv<4, true>(s[18]);
-  p[19] = mul_pow2_inv<5, true>(s[19]);
-  p[20] = mul_pow2_inv<6, true>(s[20]);
-  p[21] = mul_pow2_inv<7, true>(s[21]);
-  p[22] = mul_pow2_inv<9, true>(s[22]);
-  p[23] = mul_pow2_inv<24, true>(s[23]);
-}
+// Product by the constant W (canonical) with its Shoup companion.
+template <uint32_t W> struct P2Shoup { static constexpr uint32_t ws = shoup(W); };
+template <uint32_t W> LG_HD uint32_t mul_const(uint32_t x) { return mulc(x, W, P2Shoup<W>::ws); }
 
 // Partial rounds (S-box on lane 0, internal layer 1.1^T + diag).  With
 // R = s_1 + ... + s_23 carried from round to round, one round is
-//   u = S(s_0 + c),  sum = u + R,  s_0 <- sum + d_0 u,  s_i <- sum + d_i s_i,
-//   R <- 23 sum + sum_{i>=1} d_i s_i   (s_i before the update),
-// which is the same linear map; the products d_i s_i and their sum no longer
-// wait for the S-box, so a round's dependent chain is the S-box and two
-// additions.  s_1 .. s_23 stay unreduced in [0, 2p) between rounds (their
-// only consumer is the next product d_i s_i, which accepts them), saving two
-// of the three instructions of each of their additions.
-LG_HD void p2_partial_rounds(uint32_t s[24]) {
-  uint32_t R = tree_sum<23>(s + 1);
-  LG_UNROLL(LG_P2_PARTIAL_UNROLL)
-  for (int r = 0; r < 21; r++) {
-    const uint32_t u = p2_cube(add(s[0], LG_P2_PARTIAL_RK[r]));
-    uint32_t p[24];
-    p[1] = red(s[1]);  // d_1 = 1
-    p2_diag_products(s, p);
-    const uint32_t D = wide_sum<23>(p + 1);
-    const uint32_t sum = add(u, R);
-    s[0] = sub(R, u);  // sum + d_0 u with d_0 = -2
-#pragma unroll
-    for (int i = 1; i < 24; i++) s[i] = sum + p[i];
-    R = add(mulc(sum, C23, C23_SH), D);
+//   u = S(s_0 + c),  sum = u + R,  s_0 <- sum + d_0 u = R - u,
+//   s_i <- sum + d_i s_i,  R <- 23 sum + D,  D = sum_{i>=1} d_i s_i,
+// the same linear map with the products off the S-box's dependent chain.
+//
+// Eighteen of the 23 diagonal entries come in pairs (d, -d).  For the lanes
+// (a, b) of such a pair the half sum S = (a + b)/2 and the half difference
+// M = (a - b)/2 follow S <- sum + d M and M <- d S, so
+//   S(r + 1) = sum(r) + d^2 S(r - 1),
+// and the pair's share of D is 2 d M = 2 d^2 S(r - 1): one product, one
+// addition and one summand per pair and round where the two lanes took two of
+// each.  S(-1) = M(0)/d starts the recurrence; at the end a = S + M and
+// b = S - M with M(r) = d S(r - 1).
+//
+// S and the five single lanes stay unreduced in [0, 2p) between rounds (their
+// only consumer is the next product).  D and 23 sum are summed in 64 bits
+// and reduced once: T < 46 p, and with T = h 2^31 + l the value
+// l + h (2^24 - 1) = T - h p lies below 2^31 + 46 2^24 < 2p.
+//
+// What bounds it: the arithmetic pipes (no memory traffic).  2426 warp
+// instructions for the 21 rounds against 3636 for the form lane by lane, and
+// 25.1 against 38.6 SM clocks per permutation on B200.
+constexpr int P2_PAIRS = 9, P2_SINGLES = 5;
+// lanes of pair j, its entry d = 2^-k (k > 0) or the integer `num` (k = 0)
+struct P2Pair { int a, b, k; uint32_t num; };
+constexpr P2Pair p2_pair(int j) {
+  return j == 0   ? P2Pair{3, 6, 1, 0}
+         : j == 1 ? P2Pair{4, 7, 0, 3}
+         : j == 2 ? P2Pair{5, 8, 0, 4}
+         : j == 3 ? P2Pair{9, 16, 8, 0}
+         : j == 4 ? P2Pair{11, 17, 3, 0}
+         : j == 5 ? P2Pair{12, 18, 4, 0}
+         : j == 6 ? P2Pair{13, 19, 5, 0}
+         : j == 7 ? P2Pair{14, 20, 6, 0}
+                  : P2Pair{15, 23, 24, 0};
+}
+template <int J> struct P2PairC {
+  static constexpr int a = p2_pair(J).a, b = p2_pair(J).b, k = p2_pair(J).k;
+  static constexpr uint32_t d = k ? cx_pow2_inv(k, false) : p2_pair(J).num;  // canonical
+  static constexpr uint32_t d2 = cx_mulmod(d, d);
+  static constexpr uint32_t inv_2d = cx_pow(cx_mulmod(2, d), P - 2);
+  static_assert(P2_DSH_H.w[a] == d && P2_DSH_H.w[b] == P - d, "the pair's diagonal entries are d and -d");
+};
+template <int J> LG_HD uint32_t p2_mul_d(uint32_t x) {
+  if constexpr (P2PairC<J>::k) return mul_pow2_inv<P2PairC<J>::k, false>(x);
+  else return mul_const<P2PairC<J>::d>(x);
+}
+template <int J> LG_HD uint32_t p2_mul_d2(uint32_t x) {
+  constexpr int k2 = 2 * P2PairC<J>::k;
+  if constexpr (k2 && k2 <= 24) return mul_pow2_inv<k2, false>(x);
+  else return mul_const<P2PairC<J>::d2>(x);
+}
+template <int J = 0> LG_HD void p2_pairs_in(const uint32_t* s, uint32_t* cur, uint32_t* prev) {
+  if constexpr (J < P2_PAIRS) {
+    using C = P2PairC<J>;
+    const uint32_t a = s[C::a], b = s[C::b];
+    cur[J] = mul_pow2_inv<1, false>(a + b);
+    if constexpr (C::inv_2d == 1) prev[J] = sub(a, b);
+    else prev[J] = mul_const<C::inv_2d>(sub_lazy(a, b));
+    p2_pairs_in<J + 1>(s, cur, prev);
   }
+}
+template <int J = 0> LG_HD void p2_pairs_out(uint32_t* s, const uint32_t* cur, const uint32_t* prev) {
+  if constexpr (J < P2_PAIRS) {
+    using C = P2PairC<J>;
+    const uint32_t c = red(cur[J]), m = p2_mul_d<J>(prev[J]);
+    s[C::a] = add(c, m);
+    s[C::b] = sub(c, m);
+    p2_pairs_out<J + 1>(s, cur, prev);
+  }
+}
+template <int J = 0> LG_HD void p2_pairs_d2(const uint32_t* prev, uint32_t* q) {
+  if constexpr (J < P2_PAIRS) {
+    q[J] = p2_mul_d2<J>(prev[J]);
+    p2_pairs_d2<J + 1>(prev, q);
+  }
+}
+static_assert(P2_DSH_H.w[2] == 2 && P2_DSH_H.w[10] == cx_pow2_inv(2, false) && P2_DSH_H.w[21] == cx_pow2_inv(7, true) &&
+                  P2_DSH_H.w[22] == cx_pow2_inv(9, true),
+              "the single lanes 2, 10, 21, 22 (lane 1: checked above)");
+
+// One partial round.  x = s_0 + this round's key; `prev` holds S(r - 1) and
+// becomes S(r + 1); `single`: the lanes 1, 2, 10, 21, 22.
+LG_HD void p2_partial_round(uint32_t* prev, uint32_t* single, uint32_t& x, uint32_t& R, uint32_t key_next) {
+  uint32_t q[P2_PAIRS], p[P2_SINGLES];
+  p2_pairs_d2(prev, q);
+  p[0] = red(single[0]);
+  p[1] = dbl(red(single[1]));
+  p[2] = mul_pow2_inv<2, false>(single[2]);
+  p[3] = mul_pow2_inv<7, true>(single[3]);
+  p[4] = mul_pow2_inv<9, true>(single[4]);
+  const uint32_t u = p2_cube(x);
+  x = sub(add(R, key_next), u);
+  const uint32_t sum = add(u, R);
+  // two summands in [0, p) fit a word: 64-bit additions of their word sums
+  uint64_t A = (uint64_t)(q[0] + q[1]) + (q[2] + q[3]);
+  A += q[4] + q[5];
+  A += q[6] + q[7];
+  A += q[8];
+  uint64_t B = (uint64_t)(p[0] + p[1]) + (p[2] + p[3]);
+  B += p[4];
+  const uint64_t T = A + A + B + (uint64_t)sum * 23u;
+  R = red((uint32_t)(T >> 31) * 0x00ffffffu + ((uint32_t)T & 0x7fffffffu));
 #pragma unroll
-  for (int i = 1; i < 24; i++) s[i] = red(s[i]);
+  for (int j = 0; j < P2_PAIRS; j++) prev[j] = sum + q[j];
+#pragma unroll
+  for (int j = 0; j < P2_SINGLES; j++) single[j] = sum + p[j];
+}
+
+LG_HD void p2_partial_rounds(uint32_t s[24]) {
+  uint32_t cur[P2_PAIRS], prev[P2_PAIRS], single[P2_SINGLES] = {s[1], s[2], s[10], s[21], s[22]};
+  uint32_t R = tree_sum<23>(s + 1);
+  p2_pairs_in(s, cur, prev);
+  uint32_t x = add(s[0], LG_P2_PARTIAL_RK[0]);
+  // two rounds a turn, so that S(r) and S(r - 1) trade places without copies
+  LG_UNROLL(1)
+  for (int r = 0; r < 20; r += 2) {
+    p2_partial_round(prev, single, x, R, LG_P2_PARTIAL_RK[r + 1]);
+    p2_partial_round(cur, single, x, R, LG_P2_PARTIAL_RK[r + 2]);
+  }
+  p2_partial_round(prev, single, x, R, 0);
+  s[0] = x;
+  p2_pairs_out(s, prev, cur);
+  s[1] = red(single[0]);
+  s[2] = red(single[1]);
+  s[10] = red(single[2]);
+  s[21] = red(single[3]);
+  s[22] = red(single[4]);
 }
 
 LG_HD void p2_permute(uint32_t s[24]) {
   p2_external(s);
-  LG_UNROLL(LG_P2_FULL_UNROLL)
+  LG_UNROLL(1)
   for (int r = 0; r < 3; r++) p2_full_round(s, LG_P2_FULL_RK[r]);
   p2_partial_rounds(s);
-  LG_UNROLL(LG_P2_FULL_UNROLL)
+  LG_UNROLL(1)
   for (int r = 3; r < 6; r++) p2_full_round(s, LG_P2_FULL_RK[r]);
 }
 
