@@ -225,9 +225,12 @@ inline void launch_lde(Ctx& c, const std::vector<LdeLane>& lanes, uint32_t log_n
 // Poseidon2 lane mapping for a launch of `parallel` independent permutation
 // chains (leaves, nodes of one level): with at least `per_sm` of them per SM,
 // one thread per chain (fewest instructions per permutation); otherwise six
-// lanes per chain for a dependent chain six times shorter.  Measured on B200:
-// one thread per chain wins for leaf hashing and injection chains from 128
-// chains per SM, for one-permutation Merkle levels from 512 (Ctx::tune).
+// lanes per chain for a dependent chain shorter by half.  The line lies where
+// the two take the same time: 28 chains per SM (B200, 148 SMs: 4144 chains).
+// Measured, six lanes against one thread: a tree of 2^13 leaves (the level of
+// 4096 nodes) 99 / 94 us, of 2^14 (8192) 120 / 109, of 2^15 145 / 119; eight
+// chained injections of width 4096 175 / 185 us, 8192 199 / 191, 16384
+// 268 / 214 (Ctx::tune).
 inline bool p2_per_thread(const Ctx& c, uint64_t parallel, uint32_t per_sm) {
   return c.leaf_mapping == 1 || (c.leaf_mapping == 0 && parallel >= (uint64_t)c.sm_count * per_sm);
 }
@@ -395,6 +398,17 @@ inline bool build_tree(Ctx& c, TreeDev& t, bool read_root = true, const FsTail* 
     fold(nl);
     uint32_t start = nl;
     while (start > tail_w) {
+      // A level with enough nodes to occupy the GPU one thread per node runs
+      // in a launch of its own: six lanes per permutation, which the subtree
+      // launches use for their short dependent chain, reach 1.7 G
+      // permutations/s at best, one thread 4.5 (a tree of 2^20 leaves by
+      // subtree launches alone: 2.06 ms, 0.5 G/s).
+      if (p2_per_thread(c, start >> 1, c.tune.p2_node_min_per_sm)) {
+        level(start >> 1);
+        fold(start >> 1);
+        start >>= 1;
+        continue;
+      }
       // one launch reaches down to `stop`: start / sub at most, and not
       // through a level with injections above the tail, whose chains run
       // GPU-wide (fold) rather than on a block's few warps
