@@ -519,4 +519,59 @@ inline Committed commit(Ctx& c, const std::vector<GroupSpec>& gs, bool keep_coef
   return cm;
 }
 
+// ---------------------------------------------------------------- evaluations
+// Values of base lanes at zeta w_n^s from their coefficients (k_eval_lanes),
+// n = 2^logn each; `factor`: w_n^s.  Returns 6 words per lane, lane by lane;
+// zeta_d: zeta's six words on the device.
+struct EvalLane { const uint32_t* coef; uint32_t logn, factor; };
+inline DBufP eval_lanes(Ctx& c, const uint32_t* zeta_d, const std::vector<EvalLane>& lanes) {
+  std::map<std::pair<uint32_t, uint32_t>, uint32_t> index;  // (log n, factor) -> point
+  std::vector<EvalPoint> points;
+  std::vector<size_t> off;
+  std::vector<EvalLaneJob> jobs;
+  size_t words = 0;
+  uint32_t max_m = 1, max_n = 1, parts = 0;
+  for (const EvalLane& l : lanes) {
+    const uint32_t n = 1u << l.logn;
+    const auto key = std::make_pair(l.logn, l.factor);
+    auto it = index.find(key);
+    if (it == index.end()) {
+      EvalPoint p{l.factor, std::max(1u, n / EVAL_RUN), nullptr, nullptr};
+      it = index.emplace(key, (uint32_t)points.size()).first;
+      off.push_back(words);
+      words += 6 * ((size_t)EVAL_RUN + p.m);
+      max_m = std::max(max_m, p.m);
+      points.push_back(p);
+    }
+    EvalLaneJob j{l.coef, n, it->second, parts};
+    if (n > EVAL_CHUNK) parts += n / EVAL_CHUNK;
+    max_n = std::max(max_n, n);
+    jobs.push_back(j);
+  }
+  auto out = std::make_shared<DBuf>(std::max<size_t>(1, 6 * jobs.size()), c.stream);
+  if (jobs.empty()) return out;
+  auto tab = std::make_shared<DBuf>(words, c.stream);
+  for (size_t i = 0; i < points.size(); i++) {
+    points[i].lo = tab->p + off[i];
+    points[i].hi = tab->p + off[i] + 6 * EVAL_RUN;
+  }
+  auto part = std::make_shared<DBuf>(6 * std::max<size_t>(1, parts), c.stream);
+  auto pd = upload_vec(c, points);
+  auto jd = upload_vec(c, jobs);
+  c.timed("claimed_values", 0, 0, [&] {
+    constexpr uint32_t per = EVAL_POW_BLOCK * EVAL_POW_TURNS;
+    k_eval_powers<<<dim3((unsigned)points.size(), (max_m + per - 1) / per), EVAL_POW_BLOCK, 0, c.stream>>>(
+        (const EvalPoint*)pd->p, zeta_d);
+    LG_LAUNCH();
+    k_eval_lanes<<<dim3((unsigned)jobs.size(), (max_n + EVAL_CHUNK - 1) / EVAL_CHUNK), EVAL_BLOCK, 0, c.stream>>>(
+        (const EvalLaneJob*)jd->p, (const EvalPoint*)pd->p, part->p, out->p);
+    LG_LAUNCH();
+    if (parts) {
+      k_eval_sum<<<(unsigned)jobs.size(), 32, 0, c.stream>>>((const EvalLaneJob*)jd->p, part->p, out->p);
+      LG_LAUNCH();
+    }
+  });
+  return out;
+}
+
 }  // namespace lg

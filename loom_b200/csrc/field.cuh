@@ -110,6 +110,15 @@ LG_HD uint32_t mul_lazy(uint32_t a, uint32_t b) {
   const uint32_t m = (uint32_t)t * P_INV;
   return (uint32_t)(t >> 32) - umulhi32(m, P) + P;
 }
+// Sum of up to four products of values in [0, p), as a Montgomery product:
+// 4 (p - 1)^2 < 2^64, so the sum needs no reduction on the way; its high word
+// lies below 2p.
+LG_HD uint32_t mont_reduce4(uint64_t t) {
+  const uint32_t m = (uint32_t)t * P_INV;
+  const uint32_t hi = (uint32_t)(t >> 32);
+  const uint32_t d = umin(hi, hi - P) - umulhi32(m, P);
+  return umin(d, d + P);
+}
 LG_HD uint32_t to_mont(uint32_t canonical) { return mul(canonical % P, R2); }
 LG_HD uint32_t from_mont(uint32_t m) { return mul(m, 1u); }
 LG_HD uint32_t mont_pow(uint32_t a, uint64_t e) {

@@ -417,40 +417,22 @@ int lg_committed_eval(lg_ctx* ctx, const lg_committed* batch, const uint32_t zet
     Ctx& c = ctx->c;
     ArenaScope arena(&c.dev_arena);
     auto zd = upload_vec(c, std::vector<uint32_t>(zeta, zeta + 6));
-    std::vector<DotJob> jobs;
-    std::vector<DBufP> keep;
-    std::map<std::pair<uint32_t, int32_t>, const uint32_t*> zp;
+    // one evaluation per (group, polynomial lane, shift)
+    std::vector<EvalLane> lanes;
     for (size_t g = 0; g < h->cm.groups.size(); g++) {
       const LdeOut& l = h->cm.groups[g];
       if (!l.coef) throw Error(LG_ERR_UNSUPPORTED, "this batch keeps no coefficients");
-      const size_t n = (size_t)1 << l.log_n;
-      for (uint32_t si = 0; si < n_shifts; si++) {
-        auto key = std::make_pair(l.log_n, shifts[si]);
-        if (!zp.count(key)) {
-          const int64_t e = ((int64_t)shifts[si] % (int64_t)n + (int64_t)n) % (int64_t)n;
-          const uint32_t ws = mont_pow(root_of_unity_mont((int)l.log_n), (uint64_t)e);
-          auto b = std::make_shared<DBuf>(6 * n, c.stream);
-          k_e6_powers<<<(unsigned)((n + 127) / 128), 128, 0, c.stream>>>(zd->p, ws, (uint32_t)n, b->p);
-          LG_LAUNCH();
-          keep.push_back(b);
-          zp[key] = b->p;
-        }
-      }
-    }
-    // one dot product per (group, polynomial lane, shift)
-    for (size_t g = 0; g < h->cm.groups.size(); g++) {
-      const LdeOut& l = h->cm.groups[g];
-      const uint32_t n = 1u << l.log_n;
+      const int64_t n = (int64_t)1 << l.log_n;
+      std::vector<uint32_t> ws;
+      for (uint32_t si = 0; si < n_shifts; si++)
+        ws.push_back(mont_pow(root_of_unity_mont((int)l.log_n), (uint64_t)(((int64_t)shifts[si] % n + n) % n)));
       for (uint32_t lane = 0; lane < l.lanes; lane++)
         for (uint32_t si = 0; si < n_shifts; si++)
-          jobs.push_back(DotJob{l.coef->p + (size_t)lane * n, zp.at({l.log_n, shifts[si]}), n, (uint32_t)jobs.size()});
+          lanes.push_back(EvalLane{l.coef->p + ((size_t)lane << l.log_n), l.log_n, ws[si]});
     }
-    std::vector<uint32_t> dots(6 * jobs.size());
-    if (!jobs.empty()) {
-      auto jd = upload_vec(c, jobs);
-      auto od = std::make_shared<DBuf>(6 * jobs.size(), c.stream);
-      k_dot<<<(unsigned)jobs.size(), 256, 0, c.stream>>>((const DotJob*)jd->p, od->p);
-      LG_LAUNCH();
+    std::vector<uint32_t> dots(6 * lanes.size());
+    if (!lanes.empty()) {
+      auto od = eval_lanes(c, zd->p, lanes);
       uint32_t* hst = c.host_staging(dots.size());
       c.d2h(hst, od->p, dots.size());
       memcpy(dots.data(), hst, dots.size() * 4);

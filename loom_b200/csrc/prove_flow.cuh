@@ -323,36 +323,21 @@ inline void Prover::claimed_values() {
       for (uint32_t x : G.ecols) add_poly(x, true);
     }
   }
-  std::map<std::pair<uint32_t, int>, DBufP> zp;  // (log n, shift) -> powers of zeta w^shift
-  std::vector<DotJob> jobs;
+  std::vector<EvalLane> lanes;
+  std::map<std::pair<uint32_t, int>, uint32_t> factor;  // (log n, shift) -> w_n^shift
   for (auto& pt : polys)
     for (auto& pgp : pt)
       for (auto& p : pgp)
         for (int s : p.shifts) {
-          auto key = std::make_pair(p.logn, s);
-          if (!zp.count(key)) {
-            uint32_t n = 1u << p.logn;
-            // zeta w^s with zeta read from its device slot
-            const uint32_t ws = mont_pow(root_of_unity_mont((int)p.logn), (uint64_t)s);
-            auto b = std::make_shared<DBuf>(6 * (size_t)n, c.stream);
-            c.timed("claimed_values", 0, 0, [&] {
-              k_e6_powers<<<(n + 127) / 128, 128, 0, c.stream>>>(fs_slot(pg.n_rounds), ws, n, b->p);
-              LG_LAUNCH();
-            });
-            zp[key] = b;
-          }
-          uint32_t n = 1u << p.logn;
+          // zeta w^s with zeta read from its device slot
+          auto f = factor.emplace(std::make_pair(p.logn, s), 0u);
+          if (f.second) f.first->second = mont_pow(root_of_unity_mont((int)p.logn), (uint64_t)s);
           for (uint32_t w = 0; w < (p.ext ? 6u : 1u); w++)
-            jobs.push_back(DotJob{p.coef + (size_t)w * n, zp[key]->p, n, (uint32_t)jobs.size()});
+            lanes.push_back(EvalLane{p.coef + ((size_t)w << p.logn), p.logn, f.first->second});
         }
-  std::vector<uint32_t> dots(6 * jobs.size());
-  if (!jobs.empty()) {
-    auto jd = upload_vec(c, jobs);
-    auto od = std::make_shared<DBuf>(6 * jobs.size(), c.stream);
-    c.timed("claimed_values", 0, 0, [&] {
-      k_dot<<<(unsigned)jobs.size(), 256, 0, c.stream>>>((const DotJob*)jd->p, od->p);
-      LG_LAUNCH();
-    });
+  std::vector<uint32_t> dots(6 * lanes.size());
+  if (!lanes.empty()) {
+    auto od = eval_lanes(c, fs_slot(pg.n_rounds), lanes);
     // the DEEP denominators depend on zeta alone: forked after the dot
     // products, they run on the side stream while the host reads the claimed
     // values back and hashes them
