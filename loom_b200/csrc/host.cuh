@@ -320,14 +320,14 @@ struct Ctx {
     tw16[logn] = b;
     return b->p;
   }
-  // Powers of w = w_{2^logw} (logw > 11) for mul_split (ntt_large.cuh):
-  // 2^11 pairs (w^i canonical, its Shoup companion), then 2^(logw - 11)
-  // pairs for w^(2^11 i); built on the host once per size.
+  // Powers of w = w_{2^logw} for mul_split (ntt_large.cuh): 2^11 pairs (w^i
+  // canonical, its Shoup companion), then 2^(logw - 11) pairs (at least one)
+  // for w^(2^11 i); built on the host once per size.
   const uint2* split_powers(int logw) {
     auto it = tw_split.find(logw);
     if (it != tw_split.end()) return reinterpret_cast<const uint2*>(it->second->p);
-    if (logw <= 11 || logw > 30) throw Error(LG_ERR_INVALID, "split powers of an unsupported order");
-    const uint32_t nlo = 1u << 11, nhi = 1u << (logw - 11);
+    if (logw < 1 || logw > 30) throw Error(LG_ERR_INVALID, "split powers of an unsupported order");
+    const uint32_t nlo = 1u << 11, nhi = logw > 11 ? 1u << (logw - 11) : 1u;
     std::vector<uint32_t> tab(2 * (size_t)(nlo + nhi));
     const uint32_t w = root_of_unity_mont(logw);
     uint32_t x = MONT_ONE;

@@ -1339,6 +1339,59 @@ __global__ void k_fold(const uint32_t* layer, uint64_t n, const uint32_t* alpha_
   st6(next, half, i, e6_add(s, d));
 }
 
+// The same fold on rows of six words (ext.E6 arrays, one after another), as
+// callers hold them: a thread reads rows 2i and 2i + 1 (48 contiguous bytes)
+// and writes row i, so the layer crosses memory once.  x_i^-1 comes from two
+// tables that stay in L1 (mul_split, ntt_large.cuh: w_n^-e = w_n^(n - e))
+// rather than a scattered read of a table as long as the layer.  VEC: 16- and
+// 8-byte accesses (the caller's rows aligned to 16 bytes).
+// What bounds it: HBM and the integer pipes about equally (72 B and 30
+// products per output row).  2^22 rows on B200: 54 us a call, 0.42 of the
+// measured HBM rate (257 us with a copy in, a transpose, the fold, a transpose
+// back and a copy out).
+constexpr int FOLD_SPLIT = 11;
+struct FoldArgs { E6 alpha; const uint2* tw; uint32_t logn; };
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_fold_rows(const uint32_t* layer, FoldArgs a, uint32_t* next) {
+  const uint32_t half = 1u << (a.logn - 1);
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= half) return;
+  E6 p, q;
+  const uint32_t* src = layer + 12 * (uint64_t)i;
+  if constexpr (VEC) {
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(src)), y = __ldg(reinterpret_cast<const uint4*>(src) + 1),
+                z = __ldg(reinterpret_cast<const uint4*>(src) + 2);
+    p = E6{{x.x, x.y, x.z, x.w, y.x, y.y}};
+    q = E6{{y.z, y.w, z.x, z.y, z.z, z.w}};
+  } else {
+#pragma unroll
+    for (int w = 0; w < 6; w++) {
+      p.c[w] = src[w];
+      q.c[w] = src[6 + w];
+    }
+  }
+  // (p - q)/2 x^-1, then (p + q)/2 + alpha of it
+  const uint32_t e = ((1u << a.logn) - bitrev32(i, (int)a.logn - 1)) & ((1u << a.logn) - 1);
+  const uint2 lo = __ldg(a.tw + (e & ((1u << FOLD_SPLIT) - 1))), hi = __ldg(a.tw + (1u << FOLD_SPLIT) + (e >> FOLD_SPLIT));
+  E6 s, d;
+#pragma unroll
+  for (int w = 0; w < 6; w++) {
+    s.c[w] = mul_pow2_inv<1, false>(p.c[w] + q.c[w]);
+    d.c[w] = mulc(mulc_lazy(mul_pow2_inv<1, false>(sub_lazy(p.c[w], q.c[w])), lo.x, lo.y), hi.x, hi.y);
+  }
+  const E6 v = e6_add(s, e6_mul(d, a.alpha));
+  uint32_t* dst = next + 6 * (uint64_t)i;
+  if constexpr (VEC) {
+    uint2* o = reinterpret_cast<uint2*>(dst);
+    o[0] = make_uint2(v.c[0], v.c[1]);
+    o[1] = make_uint2(v.c[2], v.c[3]);
+    o[2] = make_uint2(v.c[4], v.c[5]);
+  } else {
+#pragma unroll
+    for (int w = 0; w < 6; w++) dst[w] = v.c[w];
+  }
+}
+
 // The last FRI rounds in one block: for each round j, the fold of layer j
 // with challenge j (as k_fold), the levels that enter at j + 1 (as
 // k_axpy_e6), then, unless j is the last round, layer j + 1's commitment —

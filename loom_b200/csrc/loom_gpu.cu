@@ -66,6 +66,13 @@ DBufP to_device(Ctx& c, const uint32_t* src, size_t words, int on_device) {
     LG_CK(cudaMemcpyAsync(b->p, src, words * 4, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c.stream));
   return b;
 }
+// Whether two device ranges of so many words share no byte: then a kernel may
+// read one and write the other in place of a staged copy.
+bool disjoint(const uint32_t* a, size_t na, const uint32_t* b, size_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x + 4 * na <= y || y + 4 * nb <= x;
+}
+bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 void from_device(Ctx& c, uint32_t* dst, const uint32_t* src, size_t words, int on_device) {
   LG_CK(cudaMemcpyAsync(dst, src, words * 4, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, c.stream));
   LG_CK(cudaStreamSynchronize(c.stream));
@@ -713,23 +720,27 @@ int lg_fri_fold(lg_ctx* ctx, const uint32_t* layer, uint64_t n, const uint32_t a
   return guarded(ctx, [&] {
     Ctx& c = ctx->c;
     if (!layer || !out || !alpha || n < 2 || (n & (n - 1)) || n > (1ull << 24)) throw Error(LG_ERR_INVALID, "bad arguments");
-    int logn = 0;
-    while ((1ull << logn) < n) logn++;
-    auto a = to_device(c, layer, 6 * n, on_device);
-    auto soa = std::make_shared<DBuf>(6 * n, c.stream);
-    k_aos_to_soa<<<(unsigned)((6 * n + 255) / 256), 256, 0, c.stream>>>(a->p, n, 6, soa->p);
-    LG_LAUNCH();
-    auto nx = std::make_shared<DBuf>(3 * n, c.stream);
-    auto al = upload_vec(c, std::vector<uint32_t>(alpha, alpha + 6));
-    const uint32_t* tw = c.twiddles(logn);
+    FoldArgs a{};
+    while ((1ull << a.logn) < n) a.logn++;
+    for (int w = 0; w < 6; w++) a.alpha.c[w] = alpha[w];
+    a.tw = c.split_powers((int)a.logn);
+    // device rows are read and written in place, unless they overlap
+    DBufP src, dst;
+    const bool direct = on_device && disjoint(layer, 6 * n, out, 3 * n);
+    if (!direct) {
+      src = to_device(c, layer, 6 * n, on_device);
+      dst = std::make_shared<DBuf>(3 * n, c.stream);
+    }
+    const uint32_t* in = direct ? layer : src->p;
+    uint32_t* to = direct ? out : dst->p;
     c.timed("fri_fold", 36.0 * n, 0, [&] {
-      k_fold<<<(unsigned)((n / 2 + 255) / 256), 256, 0, c.stream>>>(soa->p, n, al->p, tw, inv(to_mont(2)), nx->p);
+      const unsigned blocks = (unsigned)((n / 2 + 255) / 256);
+      if (aligned16(in) && aligned16(to)) k_fold_rows<true><<<blocks, 256, 0, c.stream>>>(in, a, to);
+      else k_fold_rows<false><<<blocks, 256, 0, c.stream>>>(in, a, to);
       LG_LAUNCH();
     });
-    auto aos = std::make_shared<DBuf>(3 * n, c.stream);
-    k_soa_to_aos<<<(unsigned)((3 * n + 255) / 256), 256, 0, c.stream>>>(nx->p, n / 2, 6, aos->p);
-    LG_LAUNCH();
-    from_device(c, out, aos->p, 3 * n, on_device);
+    if (direct) LG_CK(cudaStreamSynchronize(c.stream));
+    else from_device(c, out, dst->p, 3 * n, on_device);
   });
 }
 
