@@ -14,7 +14,7 @@
 #include <mutex>
 
 #include "../../include/loom_gpu.h"
-#include "field.cuh"
+#include "scan.cuh"
 
 namespace lg {
 // Kernel launch counter of the library (lg_kernel_launches), defined with the
@@ -27,76 +27,13 @@ namespace {
 using namespace lg;
 
 constexpr uint64_t NOALLOC_GP_MAX_ROWS = 1ull << 22;  // the largest loom module (2^22 rows)
-constexpr int NA_THREADS = 256, NA_PER_THREAD = 8, NA_TILE = NA_THREADS * NA_PER_THREAD;
-constexpr uint32_t NA_MAX_TILES = (uint32_t)(NOALLOC_GP_MAX_ROWS / NA_TILE);  // 2048
+constexpr uint32_t NA_MAX_TILES = (uint32_t)(NOALLOC_GP_MAX_ROWS / GP_TILE_L);  // 2048
+static_assert((1u << 16) / GP_TILE_S <= NA_MAX_TILES && (1u << 18) / GP_TILE_M <= NA_MAX_TILES, "tiles fit the scratch");
 
 // Tile totals [0, 6 * NA_MAX_TILES) and their exclusive prefix products
 // [6 * NA_MAX_TILES, 12 * NA_MAX_TILES): 96 KiB.  Every word a call reads is
 // written earlier in the same call, so nothing has to be cleared.
 static __device__ __align__(256) uint32_t g_gp_scratch[12 * NA_MAX_TILES];
-
-__device__ __forceinline__ E6 ld_row(const uint32_t* p, uint64_t i) {
-  E6 r;
-  for (int w = 0; w < 6; w++) r.c[w] = p[6 * i + w];
-  return r;
-}
-__device__ __forceinline__ void st_row(uint32_t* p, uint64_t i, const E6& v) {
-  for (int w = 0; w < 6; w++) p[6 * i + w] = v.c[w];
-}
-
-__global__ void k_na_ratio(const uint32_t* num, const uint32_t* den, uint64_t n, uint32_t* out) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  st_row(out, i, e6_mul(ld_row(num, i), e6_inv(ld_row(den, i))));
-}
-
-// In-place exclusive product scan inside each tile of NA_TILE rows; the tile
-// product goes to totals[6 t + w].
-__global__ void k_na_scan(uint32_t* x, uint64_t n, uint32_t* totals) {
-  __shared__ E6 part[NA_THREADS];
-  const uint64_t base = (uint64_t)blockIdx.x * NA_TILE + (uint64_t)threadIdx.x * NA_PER_THREAD;
-  E6 v[NA_PER_THREAD];
-  E6 acc = e6_one();
-  for (int i = 0; i < NA_PER_THREAD; i++) {
-    v[i] = acc;  // product of this thread's rows before row i
-    uint64_t idx = base + i;
-    if (idx < n) acc = e6_mul(acc, ld_row(x, idx));
-  }
-  part[threadIdx.x] = acc;
-  __syncthreads();
-  for (int off = 1; off < NA_THREADS; off <<= 1) {
-    E6 t = threadIdx.x >= (unsigned)off ? part[threadIdx.x - off] : e6_one();
-    __syncthreads();
-    if (threadIdx.x >= (unsigned)off) part[threadIdx.x] = e6_mul(part[threadIdx.x], t);
-    __syncthreads();
-  }
-  const E6 pre = threadIdx.x ? part[threadIdx.x - 1] : e6_one();
-  for (int i = 0; i < NA_PER_THREAD; i++) {
-    uint64_t idx = base + i;
-    if (idx < n) st_row(x, idx, e6_mul(pre, v[i]));
-  }
-  if (threadIdx.x == NA_THREADS - 1)
-    for (int w = 0; w < 6; w++) totals[6 * blockIdx.x + w] = part[NA_THREADS - 1].c[w];
-}
-
-__global__ void k_na_prefix(const uint32_t* totals, uint32_t nt, uint32_t* pre) {
-  E6 acc = e6_one();
-  for (uint32_t t = 0; t < nt; t++) {
-    for (int w = 0; w < 6; w++) pre[6 * t + w] = acc.c[w];
-    E6 v;
-    for (int w = 0; w < 6; w++) v.c[w] = totals[6 * t + w];
-    acc = e6_mul(acc, v);
-  }
-}
-
-__global__ void k_na_apply(uint32_t* x, uint64_t n, const uint32_t* pre) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint64_t t = i / NA_TILE;
-  E6 p;
-  for (int w = 0; w < 6; w++) p.c[w] = pre[6 * t + w];
-  st_row(x, i, e6_mul(p, ld_row(x, i)));
-}
 
 // Device address of g_gp_scratch, looked up once per device with that
 // device current (host code cannot use the symbol's name as a pointer).
@@ -131,14 +68,21 @@ extern "C" int lg_grand_product_noalloc(const uint32_t* num, const uint32_t* den
   int rc = scratch_for_current_device(&scratch);
   if (rc != LG_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  const uint32_t nt = (uint32_t)((n + NA_TILE - 1) / NA_TILE);
+  const uint32_t tile = gp_tile(n), nt = (uint32_t)((n + tile - 1) / tile);
   uint32_t* totals = scratch;
   uint32_t* pre = scratch + 6 * NA_MAX_TILES;
-  const unsigned g = (unsigned)((n + 255) / 256);
-  k_na_ratio<<<g, 256, 0, st>>>(num, den, n, out);
-  k_na_scan<<<nt, NA_THREADS, 0, st>>>(out, n, totals);
-  k_na_prefix<<<1, 1, 0, st>>>(totals, nt, pre);
-  k_na_apply<<<g, 256, 0, st>>>(out, n, pre);
+  with_gp_shape(n, [&](auto TC, auto RC) {
+    constexpr int T = decltype(TC)::value, R = decltype(RC)::value;
+    auto go = [&](auto V) {
+      constexpr bool VEC = decltype(V)::value;
+      k_rows_ratio<T, R, VEC><<<nt, T, 0, st>>>(num, den, n, out);
+      k_rows_scan<T, R, VEC, false><<<nt, T, 0, st>>>(nullptr, nullptr, n, out, totals);
+      k_rows_prefix<256><<<1, 256, 0, st>>>(totals, nt, pre);
+      k_rows_apply<T, R, VEC, true><<<nt, T, 0, st>>>(out, n, pre);
+    };
+    if (((uintptr_t)num | (uintptr_t)den | (uintptr_t)out) & 7) go(std::false_type{});
+    else go(std::true_type{});
+  });
   note_launches(4);
   return cudaGetLastError() == cudaSuccess ? LG_OK : LG_ERR_CUDA;
 }

@@ -7,6 +7,7 @@
 #include "field.cuh"
 #include "p2_coop.cuh"
 #include "ntt16.cuh"
+#include "scan.cuh"
 
 namespace lg {
 
@@ -784,57 +785,44 @@ struct ScanJob {
   uint32_t* end = nullptr; // ... and its last value written here (6 words)
 };
 
-// The scans run over products (grand products) or sums (logup running sums).
-template <bool SUM> __device__ __forceinline__ E6 scan_id() { return SUM ? e6_zero() : e6_one(); }
-template <bool SUM> __device__ __forceinline__ E6 scan_op(const E6& a, const E6& b) {
-  return SUM ? e6_add(a, b) : e6_mul(a, b);
-}
-
 template <bool SUM = false>
-__global__ void k_scan_tiles(const ScanJob* jobs) {
-  __shared__ E6 part[SCAN_BLOCK];
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(const ScanJob* jobs) {
+  __shared__ E6 sh[SCAN_BLOCK / 32];
   const ScanJob& J = jobs[blockIdx.y];
   if (blockIdx.x >= J.nt) return;
   const uint64_t n = J.n;
   const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_PER_THREAD;
   E6 acc = scan_id<SUM>();
   E6 v[SCAN_PER_THREAD];
+#pragma unroll
   for (int i = 0; i < SCAN_PER_THREAD; i++) {
-    uint64_t idx = base + i;
-    v[i] = idx < n ? ld6(J.x, n, idx) : scan_id<SUM>();
-    acc = scan_op<SUM>(acc, v[i]);
+    if (base + i < n) acc = scan_op<SUM>(acc, ld6(J.x, n, base + i));
     v[i] = acc;
   }
-  part[threadIdx.x] = acc;
-  __syncthreads();
-  for (int off = 1; off < SCAN_BLOCK; off <<= 1) {
-    E6 t = threadIdx.x >= (unsigned)off ? part[threadIdx.x - off] : scan_id<SUM>();
-    __syncthreads();
-    if (threadIdx.x >= (unsigned)off) part[threadIdx.x] = scan_op<SUM>(part[threadIdx.x], t);
-    __syncthreads();
-  }
-  E6 pre = threadIdx.x ? part[threadIdx.x - 1] : scan_id<SUM>();
-  for (int i = 0; i < SCAN_PER_THREAD; i++) {
-    uint64_t idx = base + i;
-    if (idx < n) st6(J.x, n, idx, scan_op<SUM>(pre, v[i]));
-  }
-  if (threadIdx.x == SCAN_BLOCK - 1)
-    for (int w = 0; w < 6; w++) J.totals[w * J.nt + blockIdx.x] = part[SCAN_BLOCK - 1].c[w];
+  E6 total;
+  const E6 pre = block_scan<SUM, SCAN_BLOCK>(acc, sh, total);
+#pragma unroll
+  for (int i = 0; i < SCAN_PER_THREAD; i++)
+    if (base + i < n) st6(J.x, n, base + i, scan_op<SUM>(pre, v[i]));
+  if (threadIdx.x < 6) J.totals[threadIdx.x * J.nt + blockIdx.x] = total.c[threadIdx.x];
 }
 
-// Exclusive prefix (products or sums) of the tile totals (one thread per
-// job; nt is n / 2048).
+// Exclusive prefix (products or sums) of the tile totals, one block per job
+// (nt is n / 2048: a thread alone took 34 us for the 128 tiles of 2^18 rows).
+constexpr int PREFIX_BLOCK = 64;
 template <bool SUM = false>
-__global__ void k_tile_prefix(const ScanJob* jobs, uint32_t n_jobs) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_jobs) return;
-  const ScanJob& J = jobs[i];
+__global__ void __launch_bounds__(PREFIX_BLOCK) k_tile_prefix(const ScanJob* jobs) {
+  __shared__ E6 sh[PREFIX_BLOCK / 32];
+  const ScanJob& J = jobs[blockIdx.x];
+  const uint32_t per = (J.nt + PREFIX_BLOCK - 1) / PREFIX_BLOCK, first = threadIdx.x * per;
   E6 acc = scan_id<SUM>();
-  for (uint32_t t = 0; t < J.nt; t++) {
+  for (uint32_t t = first; t < first + per && t < J.nt; t++) acc = scan_op<SUM>(acc, ld6(J.totals, J.nt, t));
+  E6 total;
+  acc = block_scan<SUM, PREFIX_BLOCK>(acc, sh, total);
+  for (uint32_t t = first; t < first + per && t < J.nt; t++) {
+#pragma unroll
     for (int w = 0; w < 6; w++) J.pre[t * 6 + w] = acc.c[w];
-    E6 v;
-    for (int w = 0; w < 6; w++) v.c[w] = J.totals[w * J.nt + t];
-    acc = scan_op<SUM>(acc, v);
+    acc = scan_op<SUM>(acc, ld6(J.totals, J.nt, t));
   }
 }
 

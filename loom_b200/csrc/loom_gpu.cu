@@ -30,13 +30,6 @@ __global__ void k_soa_to_aos(const uint32_t* in, uint64_t n, uint32_t lanes, uin
   out[i] = in[w * n + row];
 }
 
-__global__ void k_e6_div_soa(const uint32_t* num, const uint32_t* den, uint64_t n, uint32_t* out) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  E6 a = ld6(num, n, i), b = ld6(den, n, i);
-  st6(out, n, i, e6_mul(a, e6_inv(b)));
-}
-
 template <class F> int guarded(lg_ctx* ctx, F f) {
   if (!ctx) return LG_ERR_INVALID;
   try {
@@ -748,31 +741,48 @@ int lg_grand_product(lg_ctx* ctx, const uint32_t* num, const uint32_t* den, uint
   return guarded(ctx, [&] {
     Ctx& c = ctx->c;
     if (!num || !den || !out || n == 0) throw Error(LG_ERR_INVALID, "bad arguments");
-    auto na = to_device(c, num, 6 * n, on_device), da = to_device(c, den, 6 * n, on_device);
-    auto ns = std::make_shared<DBuf>(6 * n, c.stream), ds = std::make_shared<DBuf>(6 * n, c.stream);
-    unsigned g6 = (unsigned)((6 * n + 255) / 256), g1 = (unsigned)((n + 255) / 256);
-    k_aos_to_soa<<<g6, 256, 0, c.stream>>>(na->p, n, 6, ns->p);
-    LG_LAUNCH();
-    k_aos_to_soa<<<g6, 256, 0, c.stream>>>(da->p, n, 6, ds->p);
-    LG_LAUNCH();
-    auto ratio = std::make_shared<DBuf>(6 * n, c.stream);
-    k_e6_div_soa<<<g1, 256, 0, c.stream>>>(ns->p, ds->p, n, ratio->p);
-    LG_LAUNCH();
-    uint32_t nt = (uint32_t)((n + SCAN_TILE - 1) / SCAN_TILE);
-    auto totals = std::make_shared<DBuf>(6 * (size_t)nt, c.stream), pre = std::make_shared<DBuf>(6 * (size_t)nt, c.stream);
-    auto res = std::make_shared<DBuf>(6 * n, c.stream);
-    std::vector<ScanJob> sj = {ScanJob{ratio->p, n, totals->p, pre->p, res->p, nt}};
-    auto sd = upload_vec(c, sj);
-    k_scan_tiles<<<dim3(nt, 1), SCAN_BLOCK, 0, c.stream>>>((const ScanJob*)sd->p);
-    LG_LAUNCH();
-    k_tile_prefix<<<1, 64, 0, c.stream>>>((const ScanJob*)sd->p, 1);
-    LG_LAUNCH();
-    k_gp_finish<<<dim3(g1, 1), 256, 0, c.stream>>>((const ScanJob*)sd->p);
-    LG_LAUNCH();
-    auto aos = std::make_shared<DBuf>(6 * n, c.stream);
-    k_soa_to_aos<<<g6, 256, 0, c.stream>>>(res->p, n, 6, aos->p);
-    LG_LAUNCH();
-    from_device(c, out, aos->p, 6 * n, on_device);
+    // device rows are read and written in place: a tile's rows are read before
+    // they are written, so `out` may be `num` or `den` itself but may not
+    // overlap them in another way
+    auto apart = [&](const uint32_t* p) { return p == out || disjoint(p, 6 * n, out, 6 * n); };
+    const bool direct = on_device && apart(num) && apart(den);
+    DBufP na, da, res;
+    if (!direct) {
+      na = to_device(c, num, 6 * n, on_device);
+      da = to_device(c, den, 6 * n, on_device);
+      res = std::make_shared<DBuf>(6 * n, c.stream);
+    }
+    const uint32_t *a = direct ? num : na->p, *d = direct ? den : da->p;
+    uint32_t* x = direct ? out : res->p;
+    const uint32_t tile = gp_tile(n), nt = (uint32_t)((n + tile - 1) / tile);
+    auto totals = std::make_shared<DBuf>(6 * (size_t)nt, c.stream);
+    // with more tiles than this, multiplying the totals anew in every block
+    // would cost more than a launch for their prefix products
+    const bool separate = nt > 1024;
+    DBufP pre = separate ? std::make_shared<DBuf>(6 * (size_t)nt, c.stream) : nullptr;
+    c.timed("grand_product", 0, 0, [&] {
+      with_gp_shape(n, [&](auto TC, auto RC) {
+        constexpr int T = decltype(TC)::value, R = decltype(RC)::value;
+        auto go = [&](auto V) {
+          constexpr bool VEC = decltype(V)::value;
+          k_rows_scan<T, R, VEC, true><<<nt, T, 0, c.stream>>>(a, d, n, x, totals->p);
+          LG_LAUNCH();
+          if (separate) {
+            k_rows_prefix<256><<<1, 256, 0, c.stream>>>(totals->p, nt, pre->p);
+            LG_LAUNCH();
+            k_rows_apply<T, R, VEC, true><<<nt, T, 0, c.stream>>>(x, n, pre->p);
+            LG_LAUNCH();
+          } else if (nt > 1) {
+            k_rows_apply<T, R, VEC, false><<<nt, T, 0, c.stream>>>(x, n, totals->p);
+            LG_LAUNCH();
+          }
+        };
+        if (((uintptr_t)a | (uintptr_t)d | (uintptr_t)x) & 7) go(std::false_type{});
+        else go(std::true_type{});
+      });
+    });
+    if (direct) LG_CK(cudaStreamSynchronize(c.stream));
+    else from_device(c, out, x, 6 * n, on_device);
   });
 }
 

@@ -913,7 +913,7 @@ struct Prover {
         LG_LAUNCH();
         k_scan_tiles<true><<<dim3(max_nt, (unsigned)count), SCAN_BLOCK, 0, c.stream>>>((const ScanJob*)sd->p);
         LG_LAUNCH();
-        k_tile_prefix<true><<<(unsigned)((count + 63) / 64), 64, 0, c.stream>>>((const ScanJob*)sd->p, (uint32_t)count);
+        k_tile_prefix<true><<<(unsigned)count, PREFIX_BLOCK, 0, c.stream>>>((const ScanJob*)sd->p);
         LG_LAUNCH();
         k_logup_finish<<<dim3((max_n + 255) / 256, (unsigned)count), 256, 0, c.stream>>>((const ScanJob*)sd->p,
                                                                                          (const LogupFinish*)fd->p);
@@ -1046,7 +1046,7 @@ struct Prover {
         }
         k_scan_tiles<<<dim3(max_nt, (unsigned)count), SCAN_BLOCK, 0, c.stream>>>((const ScanJob*)sd->p);
         LG_LAUNCH();
-        k_tile_prefix<<<(unsigned)((count + 63) / 64), 64, 0, c.stream>>>((const ScanJob*)sd->p, (uint32_t)count);
+        k_tile_prefix<<<(unsigned)count, PREFIX_BLOCK, 0, c.stream>>>((const ScanJob*)sd->p);
         LG_LAUNCH();
         k_gp_finish<<<dim3((max_n + 255) / 256, (unsigned)count), 256, 0, c.stream>>>((const ScanJob*)sd->p);
         LG_LAUNCH();
