@@ -174,6 +174,19 @@ LG_HD E6 e6_mul(const E6& x, const E6& y) {
   s2(r, 2, e2_add(t02, v1));
   return r;
 }
+// x u and x v: multiplication by basis elements, additions only
+LG_HD E6 e6_mul_u(const E6& x) {
+  E6 r;
+  for (int i = 0; i < 3; i++) s2(r, i, E2{triple(x.c[2 * i + 1]), x.c[2 * i]});
+  return r;
+}
+LG_HD E6 e6_mul_v(const E6& x) {
+  E6 r;
+  s2(r, 0, e2_mul_xi(g2(x, 2)));
+  s2(r, 1, g2(x, 0));
+  s2(r, 2, g2(x, 1));
+  return r;
+}
 LG_HD E6 e6_sqr(const E6& x) { return e6_mul(x, x); }
 
 // (c0, c1, c2) / (a0 c0 + xi (a2 c1 + a1 c2)) with c0 = a0^2 - xi a1 a2,

@@ -1187,16 +1187,24 @@ __global__ void __launch_bounds__(32) k_eval_sum(const EvalLaneJob* jobs, const 
 // evaluated on the 4n LDE rows instead of the n trace rows and re-encoded:
 // DQ has degree < n, so both give the same codeword).
 constexpr int DEEP_MAX_POINTS = 4;
-struct DeepBundle { const uint32_t* lane0; uint64_t lane_stride; uint32_t ext; uint32_t mask; E6 scale; };
+// Every polynomial enters as base lanes with an E6 coefficient each (an
+// extension polynomial as its six lanes, alpha^i times the basis elements), so
+// a row's sum is one dot product over the lanes of the class.  Lanes are
+// sorted by the set of points they are opened at (`mask`) and padded to whole
+// quads of one mask with zero coefficients: four products are summed before
+// each reduction (mont_reduce4).
+struct DeepLane { const uint32_t* p; uint32_t c[6]; uint32_t mask, pad; };
 struct DeepJob {
-  const DeepBundle* bundles;
-  uint32_t n_bundles;
+  const DeepLane* lanes;
+  uint32_t n_lanes;     // a multiple of four
   uint32_t n_points;
   E6 z[DEEP_MAX_POINTS];
   E6 a[DEEP_MAX_POINTS];
+  const uint32_t* a_dev;  // a[0] on the device instead (null: a)
   int logn4;            // log2 of the LDE size
+  uint32_t vec;         // lanes aligned to the rows a thread takes
   const uint32_t* tw;   // w_4n^j table
-  uint32_t* out;        // 6 lanes, lane stride 4n
+  uint32_t* out;        // 6 lanes, lane stride 4n; or rows of six words
   const uint32_t* den;  // 1/(z_s - x) from k_deep_den (null: computed here)
 };
 
@@ -1234,57 +1242,222 @@ __global__ void k_deep_den(const DenJob* jobs, const uint32_t* zeta_w) {
   }
   put(0, inv_run);
 }
-__global__ void k_deep(const DeepJob* jobs) {
+// ROWS consecutive rows of a lane.
+template <int ROWS> __device__ __forceinline__ void ld_rows(const uint32_t* p, bool vec, uint32_t* x) {
+  if (vec) {
+    if constexpr (ROWS == 4) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+      x[0] = v.x;
+      x[1] = v.y;
+      x[2] = v.z;
+      x[3] = v.w;
+    } else {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      x[0] = v.x;
+      x[1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) x[i] = __ldg(p + i);
+  }
+}
+
+// 1/(z - x_i) for ROWS values x_i: the parts of e6_inv that hold z's second
+// and third coefficient are the same for all of them, and the base-field
+// inversions share one (Montgomery's trick; a zero norm, z = x_i, gives 0 as
+// inv(0) does).
+template <int ROWS> __device__ __forceinline__ void deep_inverses(const E6& z, const uint32_t* x, E6* out) {
+  const E2 a1 = g2(z, 1), a2 = g2(z, 2);
+  const E2 k1 = e2_mul_xi(e2_mul(a1, a2)), k2 = e2_mul_xi(e2_mul(a2, a2)), k3 = e2_mul(a1, a1);
+  // t = a0 (a0^2 - 3 k1) + k4, k4 = xi (a2 k2 + a1 k3)
+  const E2 k4 = e2_mul_xi(e2_add(e2_mul(a2, k2), e2_mul(a1, k3)));
+  const E2 k13 = {triple(k1.a0), triple(k1.a1)};
+  E2 t[ROWS];
+  uint32_t norm[ROWS], pre[ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; i++) {
+    const E2 a0 = {sub(z.c[0], x[i]), z.c[1]};
+    t[i] = e2_add(e2_mul(a0, e2_sub(e2_mul(a0, a0), k13)), k4);
+    norm[i] = sub(sqr(t[i].a0), triple(sqr(t[i].a1)));
+    pre[i] = norm[i] ? norm[i] : MONT_ONE;
+    if (i) pre[i] = mul(pre[i], pre[i - 1]);
+  }
+  uint32_t run = inv(pre[ROWS - 1]);
+#pragma unroll
+  for (int i = ROWS - 1; i >= 0; i--) {
+    uint32_t ni = i ? mul(run, pre[i - 1]) : run;
+    run = mul(run, norm[i] ? norm[i] : MONT_ONE);
+    if (!norm[i]) ni = 0;
+    const E2 ti = {mul(t[i].a0, ni), mul(neg(t[i].a1), ni)};
+    const E2 a0 = {sub(z.c[0], x[i]), z.c[1]};
+    s2(out[i], 0, e2_mul(e2_sub(e2_mul(a0, a0), k1), ti));
+    s2(out[i], 1, e2_mul(e2_sub(k2, e2_mul(a0, a1)), ti));
+    s2(out[i], 2, e2_mul(e2_sub(k3, e2_mul(a0, a2)), ti));
+  }
+}
+
+// DEEP quotients, ROWS consecutive rows per thread; the lanes' pointers and
+// coefficients are staged in shared memory.  ROWMAJOR: rows of six words out,
+// one point, the denominators computed here.  NP: points held in registers
+// (at least the job's).
+// What bounds it: the integer-multiply pipe (6 wide products per lane and row).
+// 48 lanes of 2^20 rows on B200: 150 us a call (349 us lane by lane, with the
+// points' sums in local memory and a transposing pass after it).
+constexpr int DEEP_BLOCK = 128, DEEP_STAGE = 64;
+template <int NP, int ROWS, bool ROWMAJOR>
+__global__ void __launch_bounds__(DEEP_BLOCK) k_deep(const DeepJob* jobs) {
+  __shared__ __align__(16) DeepLane sh[DEEP_STAGE];
   const DeepJob& jb = jobs[blockIdx.y];
   const uint32_t big = 1u << jb.logn4;
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= big) return;
-  E6 acc[DEEP_MAX_POINTS];
-  for (uint32_t s = 0; s < jb.n_points; s++) acc[s] = jb.a[s];
-  for (uint32_t b = 0; b < jb.n_bundles; b++) {
-    DeepBundle bu = jb.bundles[b];
-    E6 v;
-    if (bu.ext) {
-      E6 px;
-      for (int w = 0; w < 6; w++) px.c[w] = bu.lane0[w * bu.lane_stride + r];
-      v = e6_mul(bu.scale, px);
-    } else {
-      v = e6_mul_base(bu.scale, bu.lane0[r]);
-    }
-    for (uint32_t s = 0; s < jb.n_points; s++)
-      if (bu.mask >> s & 1) acc[s] = e6_sub(acc[s], v);
-  }
-  const uint32_t np = jb.n_points;
-  if (jb.den) {  // the denominators are precomputed
-    E6 dq = e6_zero();
-    for (uint32_t s = 0; s < np; s++) {
-      E6 is;
+  if (blockIdx.x * (uint32_t)(DEEP_BLOCK * ROWS) >= big) return;
+  const uint32_t r = (blockIdx.x * DEEP_BLOCK + threadIdx.x) * ROWS;
+  const bool in = r < big, vec = jb.vec != 0;
+  E6 acc[NP][ROWS];
 #pragma unroll
-      for (int w = 0; w < 6; w++) is.c[w] = jb.den[(uint64_t)(6 * s + w) * big + r];
-      dq = e6_add(dq, e6_mul(acc[s], is));
+  for (int s = 0; s < NP; s++)
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) {
+      acc[s][i] = jb.a[s];
+      if (ROWMAJOR && jb.a_dev)
+#pragma unroll
+        for (int w = 0; w < 6; w++) acc[s][i].c[w] = jb.a_dev[w];
     }
-    for (int w = 0; w < 6; w++) jb.out[(uint64_t)w * big + r] = dq.c[w];
-    return;
-  }
-  uint32_t x = __ldg(jb.tw + bitrev32(r, jb.logn4));
-  // sum_s acc_s / (z_s - x) with one inversion (Montgomery's trick over the
-  // points): pre_s = d_0 ... d_s, then 1/d_s = pre_(s-1) / pre_s from the top
-  E6 d[DEEP_MAX_POINTS], pre[DEEP_MAX_POINTS];
-  for (uint32_t s = 0; s < np; s++) {
-    d[s] = jb.z[s];
-    d[s].c[0] = sub(d[s].c[0], x);
-    pre[s] = s ? e6_mul(pre[s - 1], d[s]) : d[s];
-  }
-  E6 dq = e6_zero();
-  if (np) {
-    E6 inv_run = e6_inv(pre[np - 1]);  // 1 / (d_0 ... d_(np-1))
-    for (uint32_t s = np - 1; s > 0; s--) {
-      dq = e6_add(dq, e6_mul(acc[s], e6_mul(inv_run, pre[s - 1])));
-      inv_run = e6_mul(inv_run, d[s]);
+  E6 sum[ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; i++) sum[i] = e6_zero();
+  uint32_t mask = 0;
+  auto flush = [&]() {
+#pragma unroll
+    for (int s = 0; s < NP; s++)
+      if (mask >> s & 1)
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) acc[s][i] = e6_sub(acc[s][i], sum[i]);
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) sum[i] = e6_zero();
+  };
+  for (uint32_t l0 = 0; l0 < jb.n_lanes; l0 += DEEP_STAGE) {
+    const uint32_t cnt = min((uint32_t)DEEP_STAGE, jb.n_lanes - l0);
+    constexpr uint32_t W = sizeof(DeepLane) / 4;
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < cnt * W; k += DEEP_BLOCK)
+      reinterpret_cast<uint32_t*>(sh)[k] = reinterpret_cast<const uint32_t*>(jb.lanes + l0)[k];
+    __syncthreads();
+    if (!in) continue;
+#pragma unroll 1
+    for (uint32_t q = 0; q < cnt; q += 4) {
+      if (sh[q].mask != mask) {
+        flush();
+        mask = sh[q].mask;
+      }
+      uint32_t x[4][ROWS];
+#pragma unroll
+      for (int k = 0; k < 4; k++) ld_rows<ROWS>(sh[q + k].p + r, vec, x[k]);
+#pragma unroll
+      for (int w = 0; w < 6; w += 2) {
+        uint2 c[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) c[k] = *reinterpret_cast<const uint2*>(sh[q + k].c + w);
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) {
+          uint64_t t = (uint64_t)x[0][i] * c[0].x, u = (uint64_t)x[0][i] * c[0].y;
+#pragma unroll
+          for (int k = 1; k < 4; k++) {
+            t += (uint64_t)x[k][i] * c[k].x;
+            u += (uint64_t)x[k][i] * c[k].y;
+          }
+          sum[i].c[w] = add(sum[i].c[w], mont_reduce4(t));
+          sum[i].c[w + 1] = add(sum[i].c[w + 1], mont_reduce4(u));
+        }
+      }
     }
-    dq = e6_add(dq, e6_mul(acc[0], inv_run));
   }
-  for (int w = 0; w < 6; w++) jb.out[(uint64_t)w * big + r] = dq.c[w];
+  if (!in) return;
+  flush();
+  const uint32_t np = jb.n_points;
+  E6 dq[ROWS];
+  // x of row r + i: w_4n^bitrev(r + i) = w_4n^bitrev(r) w_ROWS^bitrev(i)
+  uint32_t x[ROWS];
+  if (ROWMAJOR || !jb.den) {
+    x[0] = __ldg(jb.tw + bitrev32(r, jb.logn4));
+#pragma unroll
+    for (int i = 1; i < ROWS; i++) x[i] = __ldg(jb.tw + bitrev32(r + i, jb.logn4));
+  }
+  if constexpr (ROWMAJOR) {
+    E6 di[ROWS];
+    deep_inverses<ROWS>(jb.z[0], x, di);
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) dq[i] = e6_mul(acc[0][i], di[i]);
+    uint32_t* o = jb.out + 6 * (uint64_t)r;
+    if (vec && ROWS == 4 && ((uintptr_t)jb.out & 15) == 0) {
+      const uint32_t* v = reinterpret_cast<const uint32_t*>(dq);
+#pragma unroll
+      for (int k = 0; k < 6 * ROWS / 4; k++)
+        reinterpret_cast<uint4*>(o)[k] = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < ROWS; i++)
+#pragma unroll
+        for (int w = 0; w < 6; w++) o[6 * i + w] = dq[i].c[w];
+    }
+  } else {
+    bool pole[ROWS];  // a row at one of the points: 0, as an inversion shared by the points gives
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) {
+      dq[i] = e6_zero();
+      pole[i] = false;
+    }
+#pragma unroll
+    for (int s = 0; s < NP; s++) {
+      if (s >= np) break;
+      E6 di[ROWS];
+      if (jb.den) {
+#pragma unroll
+        for (int w = 0; w < 6; w++) {
+          uint32_t d[ROWS];
+          ld_rows<ROWS>(jb.den + (uint64_t)(6 * s + w) * big + r, vec, d);
+#pragma unroll
+          for (int i = 0; i < ROWS; i++) di[i].c[w] = d[i];
+        }
+      } else {
+        deep_inverses<ROWS>(jb.z[s], x, di);
+      }
+#pragma unroll
+      for (int i = 0; i < ROWS; i++) {
+        dq[i] = e6_add(dq[i], e6_mul(acc[s][i], di[i]));
+        pole[i] |= e6_is_zero(di[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; i++)
+      if (pole[i]) dq[i] = e6_zero();
+#pragma unroll
+    for (int w = 0; w < 6; w++) {
+      uint32_t* o = jb.out + (uint64_t)w * big + r;
+      if (vec && ROWS == 2) *reinterpret_cast<uint2*>(o) = make_uint2(dq[0].c[w], dq[ROWS - 1].c[w]);
+      else
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) o[i] = dq[i].c[w];
+    }
+  }
+}
+
+// The coefficients alpha^i of n columns in the lanes' table and
+// a = sum_i alpha^i values[i], one block.
+__global__ void __launch_bounds__(256) k_deep_coefs(E6 alpha, const uint32_t* values, uint32_t n, DeepLane* lanes,
+                                                    uint32_t* a) {
+  __shared__ E6 sh[8];
+  E6 step = alpha, v = e6_pow(alpha, threadIdx.x), sum = e6_zero();
+#pragma unroll 1
+  for (int k = 0; k < 8; k++) step = e6_sqr(step);  // alpha^256
+  for (uint32_t i = threadIdx.x; i < n; i += 256) {
+#pragma unroll
+    for (int w = 0; w < 6; w++) lanes[i].c[w] = v.c[w];
+    sum = e6_add(sum, e6_mul(v, ld6(values + 6 * (uint64_t)i, 1, 0)));
+    v = e6_mul(v, step);
+  }
+  E6 total;
+  block_scan<true, 256>(sum, sh, total);
+  if (threadIdx.x < 6) a[threadIdx.x] = total.c[threadIdx.x];
 }
 
 // ---------------------------------------------------------------- FRI

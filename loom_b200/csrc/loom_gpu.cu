@@ -23,13 +23,6 @@ __global__ void k_aos_to_soa(const uint32_t* in, uint64_t n, uint32_t lanes, uin
   uint64_t row = i / lanes, w = i % lanes;
   out[w * n + row] = in[i];
 }
-__global__ void k_soa_to_aos(const uint32_t* in, uint64_t n, uint32_t lanes, uint32_t* out) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n * lanes) return;
-  uint64_t row = i / lanes, w = i % lanes;
-  out[i] = in[w * n + row];
-}
-
 template <class F> int guarded(lg_ctx* ctx, F f) {
   if (!ctx) return LG_ERR_INVALID;
   try {
@@ -794,60 +787,45 @@ int lg_deep_quotient(lg_ctx* ctx, const uint32_t* lde, uint32_t n_cols, uint64_t
       throw Error(LG_ERR_INVALID, "bad arguments");
     int logr = 0;
     while ((1ull << logr) < rows) logr++;
-    DBufP src;
-    const uint32_t* lanes = lde;
-    if (!on_device) {
-      src = to_device(c, lde, (size_t)n_cols * rows, 0);
-      lanes = src->p;
-    }
+    // device columns are read and rows written in place, unless they overlap
+    const size_t words = (size_t)n_cols * rows;
+    const bool in_place = on_device && disjoint(lde, words, out, 6 * rows);
+    DBufP src = in_place ? nullptr : to_device(c, lde, words, on_device);
+    DBufP dst = in_place ? nullptr : std::make_shared<DBuf>(6 * rows, c.stream);
+    DBufP vals = on_device ? nullptr : to_device(c, values, 6 * (size_t)n_cols, 0);
+    const uint32_t* cols = in_place ? lde : src->p;
     E6 a, zz;
     for (int w = 0; w < 6; w++) { a.c[w] = alpha[w]; zz.c[w] = z[w]; }
-    // the claimed values are read on the host: bring them back when they live on the device
-    std::vector<uint32_t> vals_host;
-    if (on_device) {
-      vals_host.resize(6 * (size_t)n_cols);
-      LG_CK(cudaMemcpyAsync(vals_host.data(), values, vals_host.size() * 4, cudaMemcpyDeviceToHost, c.stream));
-      LG_CK(cudaStreamSynchronize(c.stream));
-      values = vals_host.data();
-    }
+    // the columns' pointers; their coefficients alpha^i are filled in on the
+    // device, next to the sum of the claimed values
+    std::vector<DeepLane> lanes((n_cols + 3) / 4 * 4, DeepLane{cols, {0, 0, 0, 0, 0, 0}, 1, 0});
+    for (uint32_t i = 0; i < n_cols; i++) lanes[i].p = cols + (size_t)i * rows;
+    auto ld = upload_vec(c, lanes);
+    auto sum = std::make_shared<DBuf>(6, c.stream);
     DeepJob jb{};
-    std::vector<DeepBundle> bundles;
-    E6 run = e6_one(), acc = e6_zero();
-    for (uint32_t i = 0; i < n_cols; i++) {
-      DeepBundle bu{};
-      bu.lane0 = lanes + (size_t)i * rows;
-      bu.lane_stride = rows;
-      bu.ext = 0;
-      bu.mask = 1;
-      bu.scale = run;
-      E6 v;
-      for (int w = 0; w < 6; w++) v.c[w] = values[6 * i + w];
-      acc = e6_add(acc, e6_mul(run, v));
-      bundles.push_back(bu);
-      run = e6_mul(run, a);
-    }
     jb.n_points = 1;
     jb.z[0] = zz;
-    jb.a[0] = acc;
-    auto bd = upload_vec(c, bundles);
-    jb.bundles = (const DeepBundle*)bd->p;
-    jb.n_bundles = n_cols;
+    jb.a_dev = sum->p;
+    jb.lanes = (const DeepLane*)ld->p;
+    jb.n_lanes = (uint32_t)lanes.size();
     jb.logn4 = logr;
+    const bool wide = rows >= 4;
+    jb.vec = ((uintptr_t)cols & (wide ? 15 : 7)) == 0;
     jb.tw = c.twiddles(logr);
-    auto soa = std::make_shared<DBuf>(6 * rows, c.stream);
-    jb.out = soa->p;
+    jb.out = in_place ? out : dst->p;
     std::vector<DeepJob> jv = {jb};
     auto jd = upload_vec(c, jv);
     c.timed("deep", (4.0 * n_cols + 24.0) * rows, 0, [&] {
-      k_deep<<<dim3((unsigned)((rows + 127) / 128), 1), 128, 0, c.stream>>>((const DeepJob*)jd->p);
+      k_deep_coefs<<<1, 256, 0, c.stream>>>(a, on_device ? values : vals->p, n_cols, (DeepLane*)ld->p, sum->p);
+      LG_LAUNCH();
+      const uint32_t per = DEEP_BLOCK * (wide ? 4 : 2);
+      const unsigned blocks = (unsigned)((rows + per - 1) / per);
+      if (wide) k_deep<1, 4, true><<<dim3(blocks, 1), DEEP_BLOCK, 0, c.stream>>>((const DeepJob*)jd->p);
+      else k_deep<1, 2, true><<<dim3(blocks, 1), DEEP_BLOCK, 0, c.stream>>>((const DeepJob*)jd->p);
       LG_LAUNCH();
     });
-    auto aos = on_device ? DBufP() : std::make_shared<DBuf>(6 * rows, c.stream);
-    uint32_t* dst = on_device ? out : aos->p;
-    k_soa_to_aos<<<(unsigned)((6 * rows + 255) / 256), 256, 0, c.stream>>>(soa->p, rows, 6, dst);
-    LG_LAUNCH();
-    if (!on_device) from_device(c, out, aos->p, 6 * rows, 0);
-    else LG_CK(cudaStreamSynchronize(c.stream));
+    if (in_place) LG_CK(cudaStreamSynchronize(c.stream));
+    else from_device(c, out, dst->p, 6 * rows, on_device);
   });
 }
 

@@ -459,8 +459,8 @@ inline void Prover::deep_codewords() {
   }
   size_t deep_off = 0;
   std::vector<DeepJob> djobs;
-  std::vector<DeepBundle> all_bundles;  // every class's bundles, one upload
-  std::vector<size_t> bundle_off;
+  std::vector<DeepLane> all_lanes;  // every class's lanes, one upload
+  std::vector<size_t> lane_off;
   std::vector<double> dbytes;
   for (size_t ci = 0; ci < classes.size(); ci++) {
     uint32_t m = classes[ci];
@@ -468,7 +468,8 @@ inline void Prover::deep_codewords() {
     size_t big = mod_n(m) << RATE_LOG;
     uint32_t w_n = root_of_unity_mont((int)logn);
     DeepJob jb{};
-    std::vector<DeepBundle> bundles;
+    std::map<uint32_t, std::vector<DeepLane>> by_mask;  // lanes opened at the same points
+    double row_bytes = 24.0;
     std::vector<E6> pts;
     std::vector<uint32_t> pts_w;  // their factors w_n^shift (first-use order, as k_deep_den)
     E6 run = e6_one();
@@ -479,12 +480,11 @@ inline void Prover::deep_codewords() {
         uint32_t lane = 0;
         for (size_t i = 0; i < polys[t][g].size(); i++) {
           const Poly& p = polys[t][g][i];
-          DeepBundle bu{};
-          bu.lane0 = l.lde->p + (size_t)lane * big;
-          bu.lane_stride = big;
-          bu.ext = p.ext;
-          bu.scale = run;
-          lane += p.ext ? 6 : 1;
+          const uint32_t* lane0 = l.lde->p + (size_t)lane * big;
+          const uint32_t n_lanes = p.ext ? 6 : 1;
+          uint32_t mask = 0;
+          lane += n_lanes;
+          row_bytes += 4.0 * n_lanes;
           for (size_t si = 0; si < p.shifts.size(); si++) {
             const uint32_t f = mont_pow(w_n, (uint64_t)p.shifts[si]);
             size_t k = 0;
@@ -496,17 +496,31 @@ inline void Prover::deep_codewords() {
               jb.a[k] = e6_zero();
             }
             jb.a[k] = e6_add(jb.a[k], e6_mul(run, cv[t][g][i][si]));
-            bu.mask |= 1u << k;
+            mask |= 1u << k;
           }
-          bundles.push_back(bu);
+          E6 vrun = run;
+          if (mask)  // an unopened polynomial adds nothing
+            for (uint32_t w = 0; w < n_lanes; w++) {
+              // run times the basis 1, u, v, u v, v^2, u v^2
+              if (w == 2 || w == 4) vrun = e6_mul_v(vrun);
+              const E6 scale = w & 1 ? e6_mul_u(vrun) : vrun;
+              DeepLane dl{lane0 + (size_t)w * big, {}, mask, 0};
+              memcpy(dl.c, scale.c, 24);
+              by_mask[mask].push_back(dl);
+            }
           run = e6_mul(run, alpha);
         }
       }
     for (size_t k = 0; k < pts.size(); k++) jb.z[k] = pts[k];
     jb.n_points = (uint32_t)pts.size();
-    bundle_off.push_back(all_bundles.size());
-    all_bundles.insert(all_bundles.end(), bundles.begin(), bundles.end());
-    jb.n_bundles = (uint32_t)bundles.size();
+    lane_off.push_back(all_lanes.size());
+    for (auto& kv : by_mask) {  // whole quads of one mask
+      auto& v = kv.second;
+      v.resize((v.size() + 3) / 4 * 4, DeepLane{v[0].p, {0, 0, 0, 0, 0, 0}, kv.first, 0});
+      all_lanes.insert(all_lanes.end(), v.begin(), v.end());
+    }
+    jb.n_lanes = (uint32_t)(all_lanes.size() - lane_off.back());
+    jb.vec = 1;
     jb.logn4 = (int)logn + RATE_LOG;
     jb.tw = c.twiddles(jb.logn4);
     deep[ci] = dbuf_slice(deep_all, deep_off, 6 * big);
@@ -514,12 +528,10 @@ inline void Prover::deep_codewords() {
     jb.out = deep[ci]->p;
     if (den_pending && ci < deep_den.size() && deep_den[ci]) jb.den = deep_den[ci]->p;
     djobs.push_back(jb);
-    double row_bytes = 24.0;
-    for (auto& bu : bundles) row_bytes += bu.ext ? 24.0 : 4.0;
     dbytes.push_back(row_bytes * big);
   }
-  auto bundles_d = upload_vec(c, all_bundles);
-  for (size_t i = 0; i < djobs.size(); i++) djobs[i].bundles = (const DeepBundle*)bundles_d->p + bundle_off[i];
+  auto lanes_d = upload_vec(c, all_lanes);
+  for (size_t i = 0; i < djobs.size(); i++) djobs[i].lanes = (const DeepLane*)lanes_d->p + lane_off[i];
   if (den_pending) {  // join the side stream's denominators
     LG_CK(cudaStreamWaitEvent(c.stream, c.join_ev, 0));
     den_pending = false;
@@ -528,10 +540,17 @@ inline void Prover::deep_codewords() {
     std::vector<DeepJob> v(djobs.begin() + first, djobs.begin() + first + count);
     uint32_t max_big = 0;
     double bytes = 0;
-    for (size_t i = first; i < first + count; i++) { max_big = std::max(max_big, 1u << djobs[i].logn4); bytes += dbytes[i]; }
+    uint32_t points = 1;
+    for (size_t i = first; i < first + count; i++) {
+      max_big = std::max(max_big, 1u << djobs[i].logn4);
+      points = std::max(points, djobs[i].n_points);
+      bytes += dbytes[i];
+    }
     auto jd = upload_vec(c, v);
     c.timed("deep", bytes, 0, [&] {
-      k_deep<<<dim3((max_big + 127) / 128, (unsigned)count), 128, 0, c.stream>>>((const DeepJob*)jd->p);
+      const dim3 grid((max_big + 2 * DEEP_BLOCK - 1) / (2 * DEEP_BLOCK), (unsigned)count);
+      if (points <= 2) k_deep<2, 2, false><<<grid, DEEP_BLOCK, 0, c.stream>>>((const DeepJob*)jd->p);
+      else k_deep<DEEP_MAX_POINTS, 2, false><<<grid, DEEP_BLOCK, 0, c.stream>>>((const DeepJob*)jd->p);
       LG_LAUNCH();
     });
   };
