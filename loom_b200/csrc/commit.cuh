@@ -278,23 +278,6 @@ struct LdeOut {
   uint32_t lanes = 0, log_n = 0;
 };
 
-// LDE of `src` lanes (all of 2^log_n rows) into one buffer (used by lg_rs_encode).
-inline LdeOut lde_lanes(Ctx& c, const std::vector<const uint32_t*>& src, uint32_t log_n, bool from_coeffs,
-                        bool keep_coef) {
-  check_ntt_size((int)log_n);
-  LdeOut r;
-  r.lanes = (uint32_t)src.size();
-  r.log_n = log_n;
-  size_t n = (size_t)1 << log_n;
-  r.lde = std::make_shared<DBuf>(src.size() * (n << RATE_LOG), c.stream);
-  if (keep_coef) r.coef = std::make_shared<DBuf>(src.size() * n, c.stream);
-  std::vector<LdeLane> lanes;
-  for (size_t i = 0; i < src.size(); i++)
-    lanes.push_back(LdeLane{src[i], r.lde->p + i * (n << RATE_LOG), keep_coef ? r.coef->p + i * n : nullptr});
-  launch_lde(c, lanes, log_n, from_coeffs);
-  return r;
-}
-
 // ---------------------------------------------------------------- trees
 struct TreeDev {
   DBufP nodes;                        // 2 * n_leaves digests, 1-indexed

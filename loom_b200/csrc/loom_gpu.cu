@@ -649,11 +649,20 @@ int lg_rs_encode(lg_ctx* ctx, const uint32_t* in, uint64_t n_rows, uint32_t n_co
     if (!in || !out || n_rows < 2 || (n_rows & (n_rows - 1))) throw Error(LG_ERR_INVALID, "bad arguments");
     uint32_t logn = 0;
     while ((1ull << logn) < n_rows) logn++;
-    auto src = to_device(c, in, n_rows * n_cols, on_device);
-    std::vector<const uint32_t*> lanes;
-    for (uint32_t i = 0; i < n_cols; i++) lanes.push_back(src->p + (size_t)i * n_rows);
-    LdeOut l = lde_lanes(c, lanes, logn, false, false);
-    from_device(c, out, l.lde->p, (size_t)n_cols * (n_rows << RATE_LOG), on_device);
+    // device columns are encoded in place of staged copies, unless they overlap
+    // or the output is not aligned to the transforms' 16-byte stores
+    const size_t words = n_rows * n_cols;
+    const bool direct = on_device && aligned16(out) && disjoint(in, words, out, words << RATE_LOG);
+    DBufP src = direct ? nullptr : to_device(c, in, words, on_device);
+    DBufP dst = direct ? nullptr : std::make_shared<DBuf>(words << RATE_LOG, c.stream);
+    const uint32_t* from = direct ? in : src->p;
+    uint32_t* to = direct ? out : dst->p;
+    std::vector<LdeLane> lanes;
+    for (size_t i = 0; i < n_cols; i++)
+      lanes.push_back(LdeLane{from + i * n_rows, to + i * (n_rows << RATE_LOG), nullptr});
+    launch_lde(c, lanes, logn, false);
+    if (direct) LG_CK(cudaStreamSynchronize(c.stream));
+    else from_device(c, out, to, words << RATE_LOG, on_device);
   });
 }
 
@@ -691,7 +700,15 @@ int lg_merkle_root(lg_ctx* ctx, const uint32_t* leaves, uint64_t n_leaves, uint3
     size_t off = 0;
     for (uint32_t k = 0; k < n_inj; k++) {
       const uint64_t w = inj_widths[k];
-      t.inj.push_back(to_device(c, inj + off, 8 * w, on_device));
+      if (on_device && aligned16(inj + off)) {  // only read: the caller's buffer as it is
+        auto b = std::make_shared<DBuf>();
+        b->p = const_cast<uint32_t*>(inj + off);
+        b->words = 8 * w;
+        b->borrowed = true;
+        t.inj.push_back(b);
+      } else {
+        t.inj.push_back(to_device(c, inj + off, 8 * w, on_device));
+      }
       uint32_t lw = 0;
       while ((1ull << lw) < w) lw++;
       t.inj_log_w.push_back(lw);
