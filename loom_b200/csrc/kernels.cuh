@@ -389,7 +389,7 @@ __global__ void k_hash_leaves(const LeafGroup* groups) {
   __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
-  L.init();
+  L.init(keys);
   const LeafGroup g = groups[blockIdx.y];
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const uint32_t k = (blockIdx.x * warps + warp) * P2_GROUPS_PER_WARP + (uint32_t)L.base / 6;
@@ -464,7 +464,7 @@ __global__ void k_merkle_level(uint32_t* nodes, uint32_t start) {
   __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
-  L.init();
+  L.init(keys);
   const uint32_t warps = blockDim.x >> 5;
   const uint32_t i = (blockIdx.x * warps + (threadIdx.x >> 5)) * P2_GROUPS_PER_WARP + (uint32_t)L.base / 6;
   merkle_node(nodes, (uint64_t)start + i, L, keys, L.lane < 30 && i < start);
@@ -474,7 +474,7 @@ __global__ void k_merkle_inject(uint32_t* nodes, uint32_t start, const uint32_t*
   __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
-  L.init();
+  L.init(keys);
   const uint32_t warps = blockDim.x >> 5;
   const uint32_t j = (blockIdx.x * warps + (threadIdx.x >> 5)) * P2_GROUPS_PER_WARP + (uint32_t)L.base / 6;
   merkle_chain(nodes, (uint64_t)start + j, j, inj, n_inj, L, keys, L.lane < 30 && j < start);
@@ -534,7 +534,7 @@ __global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, con
   __shared__ uint32_t msg[64];
   p2_load_full_keys(keys);
   P2Lane L;
-  L.init();
+  L.init(keys);
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, per = warps * P2_GROUPS_PER_WARP;
   const uint32_t nb = gridDim.x, b = blockIdx.x, slot = warp * P2_GROUPS_PER_WARP + (uint32_t)L.base / 6;
   auto fold = [&](uint32_t w) {
@@ -588,7 +588,7 @@ __global__ void k_p2_permute(uint32_t* states, uint64_t n) {
   __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
   P2Lane L;
-  L.init();
+  L.init(keys);
   const uint64_t warps = blockDim.x >> 5;
   const uint64_t i = (blockIdx.x * warps + (threadIdx.x >> 5)) * P2_GROUPS_PER_WARP + (uint64_t)L.base / 6;
   const bool active = L.lane < 30 && i < n;
@@ -1579,7 +1579,7 @@ __global__ void __launch_bounds__(1024) k_fri_tail(const FriRound* rounds, uint3
   __shared__ uint32_t msg[64];
   p2_load_full_keys(keys);  // ends with a barrier
   P2Lane L;
-  L.init();
+  L.init(keys);
   const uint32_t warps = blockDim.x >> 5, per = warps * P2_GROUPS_PER_WARP;
   const uint32_t slot = (threadIdx.x >> 5) * P2_GROUPS_PER_WARP + (uint32_t)L.base / 6;
   for (uint32_t r = 0; r < n_rounds; r++) {
@@ -1687,7 +1687,7 @@ __global__ void k_fs_challenge(const uint32_t* pre, uint32_t n_pre, const uint32
     msg[i] = i < n_pre ? pre[i] : (i < n_pre + 8 ? prev[i - n_pre] : bind[i - n_pre - 8]);
   p2_load_full_keys(keys);  // ends with a barrier
   P2Lane L;
-  L.init();
+  L.init(keys);
   uint32_t x[4] = {0, 0, 0, 0};
   for (uint32_t b = 0; b < total; b += 16) {
     const uint32_t len = min(16u, total - b);  // words 0..len of the state are overwritten
@@ -1725,7 +1725,7 @@ __global__ void __launch_bounds__(32) k_fs_chain(const FsChal* chals, uint32_t n
   }
   p2_load_full_keys(keys);  // ends with a barrier
   P2Lane L;
-  L.init();
+  L.init(keys);
   for (uint32_t i = 0; i < n_chals; i++) {
     const FsChal ch = chals[i];
     uint32_t x[4] = {0, 0, 0, 0};

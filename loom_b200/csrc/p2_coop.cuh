@@ -18,10 +18,11 @@ namespace lg {
 // p2_partial_rounds, two slots a lane (nine of the twelve taken), and the
 // single lanes, one slot a lane (five of six).  Per slot the state indices and
 // the constants with their Shoup companions; an empty slot has zeros.
-struct P2CoopShare {
+struct alignas(16) P2CoopShare {
   uint32_t a[2], b[2], single;             // state indices (24: none)
   uint32_t d2[2], d2s[2], d[2], ds[2];     // pairs: d^2 and d
   uint32_t e[2], es[2];                    // single: d and d^2
+  uint32_t pad[3];
 };
 constexpr P2CoopShare make_p2_coop_share(int lane) {
   constexpr uint32_t singles[5] = {1, 2, 10, 21, 22};
@@ -47,13 +48,23 @@ constexpr P2CoopShare make_p2_coop_share(int lane) {
   }
   return c;
 }
-struct P2CoopTable { P2CoopShare lane[6]; };
+// The full-round keys and the lanes' shares, in global memory: blocks copy them
+// to shared memory with coalesced loads.  (From constant memory, whose reads by
+// lane take a turn per address, they cost each launch about a microsecond.)
+struct P2CoopTable {
+  uint32_t key[6][24];
+  P2CoopShare lane[6];
+};
 constexpr P2CoopTable make_p2_coop_table() {
   P2CoopTable t{};
+  constexpr uint32_t rk[6][24] = LG_P2_FULL_RK_INIT;
+  for (int r = 0; r < 6; r++)
+    for (int i = 0; i < 24; i++) t.key[r][i] = rk[r][i];
   for (int i = 0; i < 6; i++) t.lane[i] = make_p2_coop_share(i);
   return t;
 }
-__constant__ P2CoopTable P2_COOP_D = make_p2_coop_table();
+__device__ const P2CoopTable P2_COOP_D = make_p2_coop_table();
+constexpr uint32_t P2C_TABLE = sizeof(P2CoopTable) / 4;
 constexpr uint32_t p2_single_sum() {
   uint64_t s = 0;
   for (int i : {1, 2, 10, 21, 22}) s += P2_DSH_H.w[i];
@@ -64,25 +75,12 @@ constexpr uint32_t P2_C1 = p2_single_sum(), P2_C1_SH = shoup(P2_C1);  // the sum
 struct P2Lane {
   int lane, base, idx;  // warp lane, first lane of the group, index in the group (0..5)
   P2CoopShare sh;       // this lane's share of the partial rounds
-  __device__ __forceinline__ void init() {
+  // `smem`: filled by p2_load_full_keys
+  __device__ __forceinline__ void init(const uint32_t* smem) {
     lane = threadIdx.x & 31;
     idx = lane % 6;
     base = lane - idx;
-    sh = P2_COOP_D.lane[idx];
-    // kept in registers: reloading them in the rounds would put a divergent
-    // constant load on the chain
-    auto keep = [](uint32_t& v) { asm volatile("" : "+r"(v)); };
-    for (int k = 0; k < 2; k++) {
-      keep(sh.d2[k]);
-      keep(sh.d2s[k]);
-      keep(sh.e[k]);
-      keep(sh.es[k]);
-      keep(sh.d[k]);
-      keep(sh.ds[k]);
-      keep(sh.a[k]);
-      keep(sh.b[k]);
-    }
-    keep(sh.single);
+    sh = reinterpret_cast<const P2CoopTable*>(smem)->lane[idx];
   }
   __device__ __forceinline__ int at(int k) const { return (base + ((idx + k) % 6)) & 31; }
   // sum over the group's six lanes, in every lane
@@ -93,14 +91,14 @@ struct P2Lane {
   }
 };
 
-// Shared memory of a block that runs cooperative permutations: the full-round
-// keys, then per warp six groups' states (five and the dummy), through which
+// Shared memory of a block that runs cooperative permutations: the table above
+// (the keys first), then per warp six groups' states (five and the dummy), through which
 // the lanes trade their chunks for the partial rounds' shares and back (25
 // words a group: the last one takes the empty slots' writes).
 constexpr uint32_t P2C_GROUP = 28;  // words per group, a multiple of four
-LG_HD constexpr uint32_t p2c_smem_words(uint32_t warps) { return 144 + warps * 6 * P2C_GROUP; }
+LG_HD constexpr uint32_t p2c_smem_words(uint32_t warps) { return P2C_TABLE + warps * 6 * P2C_GROUP; }
 __device__ __forceinline__ void p2_load_full_keys(uint32_t* smem) {
-  for (int i = threadIdx.x; i < 144; i += blockDim.x) smem[i] = (&P2_FULL_RK_D[0][0])[i];
+  for (uint32_t i = threadIdx.x; i < P2C_TABLE; i += blockDim.x) smem[i] = __ldg(reinterpret_cast<const uint32_t*>(&P2_COOP_D) + i);
   __syncthreads();
 }
 
@@ -207,7 +205,7 @@ __device__ __forceinline__ void p2c_permute(uint32_t x[4], const P2Lane& L, uint
   p2c_external(x, L);
 #pragma unroll 1
   for (int r = 0; r < 3; r++) p2c_full(x, L, smem + 24 * r);
-  p2c_partial(x, L, smem + 144 + ((threadIdx.x >> 5) * 6 + (uint32_t)L.base / 6) * P2C_GROUP);
+  p2c_partial(x, L, smem + P2C_TABLE + ((threadIdx.x >> 5) * 6 + (uint32_t)L.base / 6) * P2C_GROUP);
 #pragma unroll 1
   for (int r = 3; r < 6; r++) p2c_full(x, L, smem + 24 * r);
 }
