@@ -17,12 +17,17 @@ struct lg_ctx {
 
 namespace {
 
-__global__ void k_aos_to_soa(const uint32_t* in, uint64_t n, uint32_t lanes, uint32_t* out) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n * lanes) return;
-  uint64_t row = i / lanes, w = i % lanes;
-  out[w * n + row] = in[i];
+// Extension columns given as rows of six words, as six lanes each: a column
+// per blockIdx.y, a row per thread (so the lanes' stores are coalesced).
+struct RowsCol { const uint32_t* rows; uint32_t* lanes; uint64_t n; };
+__global__ void __launch_bounds__(256) k_rows_to_lanes(const RowsCol* cols) {
+  const RowsCol col = cols[blockIdx.y];
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (i >= col.n) return;
+  const E6 v = ((uintptr_t)col.rows & 7) == 0 ? ld_row<true>(col.rows, i) : ld_row<false>(col.rows, i);
+  st6(col.lanes, col.n, i, v);
 }
+
 template <class F> int guarded(lg_ctx* ctx, F f) {
   if (!ctx) return LG_ERR_INVALID;
   try {
@@ -308,40 +313,81 @@ namespace {
 
 // Groups of a batch given as PCS.Commit's columns (internal/fri/pcs.go:145-168):
 // rows[g] Lagrange rows, n_base[g] base columns then n_ext[g] extension
-// columns (ext.E6 rows, 6 words each) in `cols`, group by group.  Extension
-// columns are laid out as six lanes on the device.
+// columns (ext.E6 rows, 6 words each) in `cols`, group by group.  Device base
+// columns are lanes as they are (the commitment only reads them); host columns
+// go up into one buffer, neighbours in one copy; extension columns become six
+// lanes each in one launch.
 std::vector<GroupSpec> batch_groups(Ctx& c, uint32_t n_groups, const uint64_t* rows, const uint32_t* n_base,
                                     const uint32_t* n_ext, const uint32_t* const* cols, int on_device,
                                     std::vector<DBufP>& keep) {
   if (!n_groups || !rows || !n_base || !n_ext || !cols) throw Error(LG_ERR_INVALID, "null argument");
-  std::vector<GroupSpec> gs;
-  size_t ci = 0;
+  size_t words = 0, ext_words = 0, ci = 0;
   for (uint32_t g = 0; g < n_groups; g++) {
-    uint64_t n = rows[g];
+    const uint64_t n = rows[g];
     if (n < 2 || (n & (n - 1))) throw Error(LG_ERR_INVALID, "group rows must be a power of two >= 2");
+    words += n * (n_base[g] + 6 * (size_t)n_ext[g]);
+    ext_words += 6 * n * n_ext[g];
+    for (uint32_t i = 0; i < n_base[g] + n_ext[g]; i++)
+      if (!cols[ci++]) throw Error(LG_ERR_INVALID, "null column");
+  }
+  uint32_t *up = nullptr, *ext = nullptr;
+  if (!on_device) {
+    keep.push_back(std::make_shared<DBuf>(words, c.stream));
+    up = keep.back()->p;
+  }
+  if (ext_words) {
+    keep.push_back(std::make_shared<DBuf>(ext_words, c.stream));
+    ext = keep.back()->p;
+  }
+  const uint32_t* run_src = nullptr;  // a copy in the making: adjacent host columns
+  uint32_t* run_dst = nullptr;
+  size_t run_words = 0;
+  auto flush = [&] {
+    if (run_words) LG_CK(cudaMemcpyAsync(run_dst, run_src, run_words * 4, cudaMemcpyHostToDevice, c.stream));
+    run_words = 0;
+  };
+  auto device = [&](const uint32_t* col, size_t n) -> const uint32_t* {
+    if (on_device) return col;
+    uint32_t* dst = up;
+    up += n;
+    if (run_words && col == run_src + run_words) {
+      run_words += n;
+    } else {
+      flush();
+      run_src = col;
+      run_dst = dst;
+      run_words = n;
+    }
+    return dst;
+  };
+  std::vector<GroupSpec> gs;
+  std::vector<RowsCol> ext_cols;
+  uint64_t max_n = 0;
+  ci = 0;
+  for (uint32_t g = 0; g < n_groups; g++) {
+    const uint64_t n = rows[g];
     GroupSpec s;
     s.log_n = 0;
     while ((1ull << s.log_n) < n) s.log_n++;
     s.nb = n_base[g];
     s.ne = n_ext[g];
     s.from_coeffs = false;
-    for (uint32_t i = 0; i < s.nb; i++) {
-      if (!cols[ci]) throw Error(LG_ERR_INVALID, "null column");
-      auto b = to_device(c, cols[ci++], n, on_device);
-      s.lanes.push_back(b->p);
-      keep.push_back(b);
-    }
+    for (uint32_t i = 0; i < s.nb; i++) s.lanes.push_back(device(cols[ci++], n));
     for (uint32_t i = 0; i < s.ne; i++) {
-      if (!cols[ci]) throw Error(LG_ERR_INVALID, "null column");
-      auto a = to_device(c, cols[ci++], 6 * n, on_device);
-      auto b = std::make_shared<DBuf>(6 * n, c.stream);
-      k_aos_to_soa<<<(unsigned)((6 * n + 255) / 256), 256, 0, c.stream>>>(a->p, n, 6, b->p);
-      LG_LAUNCH();
-      for (int w = 0; w < 6; w++) s.lanes.push_back(b->p + (size_t)w * n);
-      keep.push_back(a);
-      keep.push_back(b);
+      ext_cols.push_back(RowsCol{device(cols[ci++], 6 * n), ext, n});
+      for (int w = 0; w < 6; w++) s.lanes.push_back(ext + (size_t)w * n);
+      ext += 6 * n;
+      max_n = std::max(max_n, n);
     }
     gs.push_back(s);
+  }
+  flush();
+  for (size_t first = 0; first < ext_cols.size(); first += 65535) {  // grid y: at most 65535 columns a launch
+    const size_t cnt = std::min<size_t>(65535, ext_cols.size() - first);
+    keep.push_back(upload_vec(c, std::vector<RowsCol>(ext_cols.begin() + first, ext_cols.begin() + first + cnt)));
+    k_rows_to_lanes<<<dim3((unsigned)((max_n + 255) / 256), (unsigned)cnt), 256, 0, c.stream>>>(
+        (const RowsCol*)keep.back()->p);
+    LG_LAUNCH();
   }
   return gs;
 }

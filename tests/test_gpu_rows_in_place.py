@@ -109,3 +109,25 @@ def test_deep_quotient_at_a_row_of_the_domain(ctx):
     z[0] = pow(w, int(f"{row:04b}"[::-1], 2), F.P)
     got = ctx.deep_quotient(lde, alpha, F.to_mont(z), values)
     assert not got[row].any() and got[[r for r in range(rows) if r != row]].any(axis=1).all()
+
+
+@pytest.mark.parametrize("shape,offset", [([(1 << 9, 3, 1), (1 << 5, 1, 2)], 0), ([(2, 1, 0), (2, 0, 1)], 1),
+                                          ([(1 << 10, 1, 1), (1 << 10, 2, 0), (1 << 15, 1, 0)], 1)])
+def test_commit_of_device_columns(ctx, shape, offset):
+    """Columns on the device, aligned or not, against the same columns on the
+    host; they are left as they were."""
+    groups, bufs, data = [], [], []
+    for gi, (n, nb, ne) in enumerate(shape):
+        base, ext = [rnd(n, 10 * gi + k) for k in range(nb)], [rnd((n, 6), 10 * gi + 5 + k) for k in range(ne)]
+        groups.append({"rows": n, "base": base, "ext": ext})
+        data += base + ext
+        bufs += [Rows(c.size, c, offset) for c in base + ext]
+    ptrs = (ctypes.c_void_p * len(bufs))(*[b.ptr().value for b in bufs])
+    rows = np.array([s[0] for s in shape], dtype=np.uint64)
+    nb, ne = (np.array([s[k] for s in shape], dtype=np.uint32) for k in (1, 2))
+    root = np.zeros(8, dtype=np.uint32)
+    ctx._check(ctx.L.lg_commit_root(ctx.h, len(shape), rows.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64)), u32(nb),
+                                    u32(ne), ptrs, 1, u32(root)))
+    assert np.array_equal(root, ctx.commit_root(groups))
+    for b, c in zip(bufs, data):
+        assert np.array_equal(b.get(c.shape), c)
