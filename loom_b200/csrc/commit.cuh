@@ -109,6 +109,38 @@ inline void big_ntt(Ctx& c, std::vector<BigNtt> jobs, int logn, bool inverse, co
   }
 }
 
+// Coset transforms of 2^logn points (logn > SMEM_NTT_MAX_LOG) by the forward
+// tree, coefficients to bit-reversed evaluations.  Jobs go in chunks whose
+// output stays in L2 between the two passes (FWD_CHUNK words).
+constexpr size_t FWD_CHUNK = (size_t)1 << 24;
+inline void big_fwd(Ctx& c, const std::vector<FwdJob>& jobs, int logn, const char* tag, double bytes_per_job) {
+  if (jobs.empty()) return;
+  const int logr = logn / 2, logc = logn - logr;
+  if (logr < 7 || logc > 11) throw Error(LG_ERR_UNSUPPORTED, "forward transform size out of range");
+  const uint2* tau = c.tree_twiddles(logn + RATE_LOG - 1);
+  auto jd = upload_vec(c, jobs);
+  const size_t smem = tile_words(logc) * 4;
+  const unsigned thr = (unsigned)std::min<size_t>(512, (size_t)1 << logc);
+  const size_t per = std::min<size_t>(65535, std::max<size_t>(1, FWD_CHUNK >> logn));
+  c.timed(tag, bytes_per_job * jobs.size(), 0, [&] {
+    for (size_t first = 0; first < jobs.size(); first += per) {
+      const unsigned cnt = (unsigned)std::min(per, jobs.size() - first);
+      const FwdJob* j = (const FwdJob*)jd->p + first;
+      with_tile_size(logc, [&](auto LC) {
+        constexpr int C_ = decltype(LC)::value;
+        allow_smem(k_fwd_cols<C_>, smem);
+        k_fwd_cols<C_><<<dim3((1u << logr) / BIG_TILE, cnt), thr, smem, c.stream>>>(j, logr, tau);
+        LG_LAUNCH();
+      });
+      with_tile_size(logr, [&](auto LR) {
+        constexpr int R_ = decltype(LR)::value;
+        k_fwd_rows<R_><<<dim3((1u << logc) / fwd_rows(R_), cnt), FWD_THREADS, 0, c.stream>>>(j, logc, tau);
+        LG_LAUNCH();
+      });
+    }
+  });
+}
+
 inline BigNtt big_job(const uint32_t* in, uint32_t* out, uint32_t c0, bool bitrev_out) {
   BigNtt j{};
   j.in = in;
@@ -127,7 +159,8 @@ inline void launch_lde(Ctx& c, const std::vector<LdeLane>& lanes, uint32_t log_n
   if ((int)log_n > SMEM_NTT_MAX_LOG) {
     DBufP tmp;
     std::vector<const uint32_t*> coef(lanes.size());
-    std::vector<BigNtt> inv_jobs, fwd_jobs;
+    std::vector<BigNtt> inv_jobs;
+    std::vector<FwdJob> fwd_jobs;
     bool need_tmp = false;
     for (auto& L : lanes) need_tmp |= !from_coeffs && !L.coef;
     if (need_tmp) tmp = std::make_shared<DBuf>(lanes.size() * n, c.stream);
@@ -139,20 +172,16 @@ inline void launch_lde(Ctx& c, const std::vector<LdeLane>& lanes, uint32_t log_n
       } else {
         uint32_t* dst = lanes[i].coef ? lanes[i].coef : tmp->p + i * n;
         inv_jobs.push_back(big_job(lanes[i].src, dst, inv(to_mont((uint32_t)n)), false));
+        inv_jobs.back().coset0 = lanes[i].out;  // <w_n> itself: the values in bit-reversed order
         coef[i] = dst;
       }
     }
     big_ntt(c, inv_jobs, (int)log_n, true, "lde", 8.0 * n);
-    const uint32_t* tw4 = c.twiddles((int)log_n + RATE_LOG);
+    const uint32_t a0 = from_coeffs ? 0 : 1;
     for (size_t i = 0; i < lanes.size(); i++)
-      for (int a = 0; a < (1 << RATE_LOG); a++) {
-        BigNtt j = big_job(coef[i], lanes[i].out + (size_t)a * n, MONT_ONE, true);
-        j.t2 = tw4;
-        j.m2_mask = (uint32_t)((n << RATE_LOG) - 1);
-        j.e2 = bitrev32((uint32_t)a, RATE_LOG);
-        fwd_jobs.push_back(j);
-      }
-    big_ntt(c, fwd_jobs, (int)log_n, false, "lde", 20.0 * n / (1 << RATE_LOG));
+      for (uint32_t a = a0; a < (1u << RATE_LOG); a++)
+        fwd_jobs.push_back(FwdJob{coef[i], lanes[i].out + (size_t)a * n, a});
+    big_fwd(c, fwd_jobs, (int)log_n, "lde", 20.0 * n / (1 << RATE_LOG));
     return;
   }
   const uint32_t* twn = c.ntt_twiddles((int)log_n);

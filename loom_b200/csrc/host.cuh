@@ -219,6 +219,8 @@ struct Ctx {
   std::map<int, DBufP> tw;       // log n -> w_n^j, j < n
   std::map<int, DBufP> tw16;     // log n -> the radix-16 passes' twiddle tables (tw16 layout, ntt16.cuh)
   std::map<int, DBufP> tw_split; // log n -> w_n's powers as two small Shoup tables (split_powers)
+  DBufP tree_tw;                 // tau[B], B < 2^tree_log (tree_twiddles)
+  int tree_log = 0;
   std::map<int, DBufP> gpow;     // log n -> g^k, k < n
   std::map<int, DBufP> ginvpow;  // log n -> g^-k, k < n
   std::map<int, DBufP> cshift;   // log n -> (g w_4n^c)^k, k < n, for c = 0..3 (4 tables back to back)
@@ -349,6 +351,22 @@ struct Ctx {
     LG_CK(cudaStreamSynchronize(stream));  // the host table goes out of scope
     tw_split[logw] = b;
     return reinterpret_cast<const uint2*>(b->p);
+  }
+  // tau of the forward tree (ntt_large.cuh) for nodes below 2^logm.  A longer
+  // table begins with the shorter ones, so one is kept: the longest asked for
+  // (the one it replaces is freed in stream order, after its last use).
+  const uint2* tree_twiddles(int logm) {
+    if (logm > tree_log) {
+      if (logm < 2 || logm > 23) throw Error(LG_ERR_INVALID, "tree twiddles of an unsupported order");
+      ArenaScope cached(nullptr);  // kept across proves: never from the arena
+      auto b = std::make_shared<DBuf>((size_t)2 << logm, stream);
+      k_fill_tree<<<((1u << logm) + 255) / 256, 256, 0, stream>>>(reinterpret_cast<uint2*>(b->p), logm,
+                                                                  root_of_unity_mont(logm + 1));
+      LG_LAUNCH();
+      tree_tw = b;
+      tree_log = logm;
+    }
+    return reinterpret_cast<const uint2*>(tree_tw->p);
   }
   // the table a transform kernel takes: tw16 for the radix-16 passes, the
   // plain powers below 16 points (radix-2 stages)

@@ -22,6 +22,15 @@ __global__ void k_fill_powers(uint32_t* out, uint64_t n, uint32_t base, uint32_t
   if (j < n) out[j] = mul(start, mont_pow(base, j));
 }
 
+// tau[B] = w^bitrev_logm(B) for B < 2^logm, w of order 2^(logm + 1): canonical
+// words with their Shoup companions (the forward tree, ntt_large.cuh).
+__global__ void k_fill_tree(uint2* out, int logm, uint32_t w) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >> logm) return;
+  const uint32_t c = from_mont(mont_pow(w, bitrev32(b, logm)));
+  out[b] = make_uint2(c, (uint32_t)(((uint64_t)c << 32) / P));
+}
+
 // ---------------------------------------------------------------- smem NTT
 // Radix-2 stages over a block-resident array A of n = 2^logn words.
 // tw: table of w_n^j (j < n) for this n; `inverse` uses w_n^-j = w_n^(n-j).
