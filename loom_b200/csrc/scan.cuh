@@ -86,55 +86,48 @@ __device__ __forceinline__ bool e6_is_zero(const E6& v) {
 constexpr uint32_t GP_TILE_S = 128, GP_TILE_M = 512, GP_TILE_L = 2048;
 inline uint32_t gp_tile(uint64_t n) { return n <= 1u << 16 ? GP_TILE_S : n <= 1u << 18 ? GP_TILE_M : GP_TILE_L; }
 
-// ratio[i] = num[i] / den[i] (0 where den[i] is 0, as e6_inv(0) = 0), in the
-// products of a thread's R rows: with A_i = num_0 .. num_(i-1) and
-// B_i = den_i .. den_(R-1), the product of the ratios before row i is
-// A_i B_i / B_0, one inversion for all R rows and three E6 products a row
-// where an inversion takes about six.  Leaves these products, times `scale`,
-// in v and returns the product of all R ratios.
-template <int R> __device__ __forceinline__ E6 ratio_products(const E6* num, const E6* den, E6* v) {
-  // v[i] = B_i from the back, then A_i B_i / B_0
-  E6 b = den[R - 1];
-  v[R - 1] = b;
-#pragma unroll
-  for (int i = R - 2; i >= 0; i--) {
-    b = e6_mul(den[i], b);
-    v[i] = b;
-  }
-  E6 a = e6_inv(b);
-  v[0] = e6_one();
-#pragma unroll
-  for (int i = 1; i < R; i++) {
-    a = e6_mul(a, num[i - 1]);
-    v[i] = e6_mul(a, v[i]);
-  }
-  return e6_mul(a, num[R - 1]);
-}
-
 // Exclusive product scan inside each tile of T R rows: of the ratios
-// num / den (RATIO; x is written), or of x in place.  Tile t's product goes to
-// totals[6 t + w].  A tile's rows are read before any of them is written.
-// What bounds it: the integer-multiply pipe (about six E6 products a row)
+// num / den (RATIO; x is written; a ratio is 0 where its denominator is 0, as
+// e6_inv(0) = 0), or of x in place.  Tile t's product goes to totals[6 t + w].
+// A tile's rows are read before any of them is written.
+//
+// With A_i = num_0 .. num_(i-1) and B_i = den_i .. den_(R-1) over a thread's
+// rows, the product of the ratios before row i is A_i B_i / B_0: one inversion
+// for all R rows and three E6 products a row, where an inversion takes about
+// six.  The denominators are taken from the back and the numerators from the
+// front, one row at a time, so only the products stay in registers.
+// What bounds it: the integer-multiply pipe (about five E6 products a row)
 // and, for few tiles, the dependent products of the scan and the inversion.
+// 512 threads an SM, 128 registers each: with both operands of every row held
+// (210 registers) 1,000,003 rows took 162 us, so 127 (start to end).
 template <int T, int R, bool VEC, bool RATIO>
-__global__ void __launch_bounds__(T) k_rows_scan(const uint32_t* num, const uint32_t* den, uint64_t n, uint32_t* x,
-                                                 uint32_t* totals) {
+__global__ void __launch_bounds__(T, 512 / T) k_rows_scan(const uint32_t* num, const uint32_t* den, uint64_t n,
+                                                          uint32_t* x, uint32_t* totals) {
   __shared__ E6 sh[T / 32];
   const uint64_t base = (uint64_t)blockIdx.x * (T * R) + (uint64_t)threadIdx.x * R;
   E6 v[R], acc;
   if constexpr (RATIO) {
-    E6 a[R], d[R];
+    uint32_t zero = 0;  // rows whose denominator is 0
+    E6 b = e6_one();
+#pragma unroll
+    for (int i = R - 1; i >= 0; i--) {
+      E6 d = base + i < n ? ld_row<VEC>(den, base + i) : e6_one();
+      if (e6_is_zero(d)) {
+        zero |= 1u << i;
+        d = e6_one();
+      }
+      b = i == R - 1 ? d : e6_mul(d, b);
+      v[i] = b;
+    }
+    acc = e6_inv(b);
+    v[0] = e6_one();
 #pragma unroll
     for (int i = 0; i < R; i++) {
-      const bool in = base + i < n;
-      a[i] = in ? ld_row<VEC>(num, base + i) : e6_one();
-      d[i] = in ? ld_row<VEC>(den, base + i) : e6_one();
-      if (e6_is_zero(d[i])) {
-        a[i] = e6_zero();
-        d[i] = e6_one();
-      }
+      if (i) v[i] = e6_mul(acc, v[i]);
+      E6 a = base + i < n ? ld_row<VEC>(num, base + i) : e6_one();
+      if (zero >> i & 1) a = e6_zero();
+      acc = e6_mul(acc, a);
     }
-    acc = ratio_products<R>(a, d, v);
   } else {
     acc = e6_one();
 #pragma unroll
@@ -155,10 +148,16 @@ __global__ void __launch_bounds__(T) k_rows_scan(const uint32_t* num, const uint
 // those products; otherwise the totals, which every block multiplies up to its
 // own tile (at most a few E6 products a thread: n / tile^2 and the block's
 // reduction), saving the launch between.
+// The block's rows are loaded before that, so the two overlap.
 template <int T, int R, bool VEC, bool PREFIX>
-__global__ void __launch_bounds__(T) k_rows_apply(uint32_t* x, uint64_t n, const uint32_t* pre) {
+__global__ void __launch_bounds__(T, 512 / T) k_rows_apply(uint32_t* x, uint64_t n, const uint32_t* pre) {
   __shared__ E6 sh[T / 32];
-  E6 p;
+  if (blockIdx.x == 0) return;  // nothing before the first tile
+  const uint64_t first = (uint64_t)blockIdx.x * (T * R) + threadIdx.x;
+  E6 v[R], p;
+#pragma unroll
+  for (int i = 0; i < R; i++)
+    if (first + i * T < n) v[i] = ld_row<VEC>(x, first + i * T);
   if constexpr (PREFIX) {
     p = ld_row<true>(pre, blockIdx.x);
   } else {
@@ -166,12 +165,9 @@ __global__ void __launch_bounds__(T) k_rows_apply(uint32_t* x, uint64_t n, const
     for (uint32_t t = threadIdx.x; t < blockIdx.x; t += T) acc = e6_mul(acc, ld_row<true>(pre, t));
     block_scan<false, T>(acc, sh, p);
   }
-  if (blockIdx.x == 0) return;  // nothing before the first tile
 #pragma unroll
-  for (int i = 0; i < R; i++) {
-    const uint64_t k = (uint64_t)blockIdx.x * (T * R) + i * T + threadIdx.x;
-    if (k < n) st_row<VEC>(x, k, e6_mul(p, ld_row<VEC>(x, k)));
-  }
+  for (int i = 0; i < R; i++)
+    if (first + i * T < n) st_row<VEC>(x, first + i * T, e6_mul(p, v[i]));
 }
 
 // Exclusive prefix products of nt tile totals, one block of T threads.
