@@ -366,7 +366,8 @@ __device__ __forceinline__ uint32_t leaf_elem(const LeafGroup& g, uint32_t idx, 
 // Kernels with a permutation per thread: built for blocks of at most 256
 // threads and 128 registers, since the permutation keeps its 24 words and the
 // products in flight in registers.  With a cap of 64 registers (1024-thread
-// blocks) the full rounds take 6.9 SM clocks instead of 6.4 (B200).
+// blocks) the full rounds take 6.9 SM clocks instead of 6.4 (B200); room for
+// more than 128 (blocks of 128, four on an SM) changes nothing.
 constexpr int P2_MAX_BLOCK = 256;
 
 // One thread per leaf: the fewest instructions per permutation, for launches
@@ -1776,12 +1777,8 @@ __global__ void k_coins_assemble(const uint32_t* slots, uint32_t n_coins, const 
 }
 
 // ---------------------------------------------------------------- openings
-// Montgomery words -> canonical values as big-endian bytes (the proof
-// encoding), in place.
-__global__ void k_proof_words(uint32_t* x, uint64_t n) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i < n) x[i] = __byte_perm(from_mont(x[i]), 0, 0x0123);
-}
+// A Montgomery word in the proof encoding: canonical, big-endian bytes.
+__device__ __forceinline__ uint32_t proof_word(uint32_t m) { return __byte_perm(from_mont(m), 0, 0x0123); }
 
 // Row pairs: for every query q and source, the rows lo and lo + 1 of each
 // lane, lo = (s_q >> shift) & ~1: row lo of every lane, then row lo + 1, at
@@ -1795,8 +1792,8 @@ __global__ void k_gather_rows(const RowSrc* srcs, uint32_t n_src, const uint32_t
   if (q >= nq || l >= s.n_lanes) return;
   uint32_t lo = (pos[q] >> s.shift) & ~1u;
   const uint32_t* p = s.lane0 + l * s.lane_stride;
-  out[q * per_q + s.off + l] = p[lo];
-  out[q * per_q + s.off + s.n_lanes + l] = p[lo + 1];
+  out[q * per_q + s.off + l] = proof_word(p[lo]);
+  out[q * per_q + s.off + s.n_lanes + l] = proof_word(p[lo + 1]);
 }
 
 // Merkle paths: siblings of leaf idx = ((s_q >> shift) >> 1), leaf level
@@ -1825,7 +1822,7 @@ __global__ void k_gather_paths(const PathSrc* srcs, const uint32_t* pos, uint32_
     uint32_t k = t - s.log_leaves;
     src = s.inj[k] + (uint64_t)(idx >> s.inj_shift[k]) * 8;
   }
-  for (int w = 0; w < 8; w++) o[w] = src[w];
+  for (int w = 0; w < 8; w++) o[w] = proof_word(src[w]);
 }
 
 // Per-query proof sections.  Every query's part of a section has the same
@@ -1845,7 +1842,7 @@ __global__ void k_assemble(const SectionSrc* secs, const uint32_t* map, const ui
   const uint32_t code = map[sc.map_off + j], kind = code >> 30, idx = code & 0x3fffffffu;
   uint32_t w;
   if (kind == SEC_COPY) {
-    w = gathered[(uint64_t)k * per_q + idx];  // already big-endian (k_proof_words)
+    w = gathered[(uint64_t)k * per_q + idx];  // already encoded (proof_word)
   } else {
     uint32_t v;
     if (kind == SEC_CONST) {
