@@ -45,16 +45,51 @@ struct SetupData {
   std::map<uint32_t, DBufP> values;            // setup column -> Lagrange values
   std::map<uint32_t, const uint32_t*> coef;    // setup column -> coefficient lane 0 (in committed)
 };
+// What a prove derives from the program descriptor alone: the parsed program
+// with its folded relations, degrees, the shift schedule and the tree layout.
+// Made by the first prove of a program, read by the later ones.
+struct Layout {
+  struct Group { uint32_t module; std::vector<uint32_t> bcols, ecols; };
+  struct TreeL { bool air; int round; std::vector<Group> groups; bool setup = false; };
+  Program pg;
+  std::vector<uint32_t> mod_order;
+  std::vector<int> fold_root, degree;
+  std::vector<bool> root_ext;
+  std::map<uint32_t, std::vector<int>> col_shifts;
+  std::vector<TreeL> trees;
+  std::vector<char> ext_of;  // per node
+  bool ready = false;        // complete: setup_layout has run through
+};
 struct ProgCache {
   std::vector<uint32_t> words;  // the program descriptor, compared in full
+  std::shared_ptr<Layout> layout;
   std::map<std::string, std::shared_ptr<CodeSet>> sites;
   std::shared_ptr<SetupData> setup;
 };
 
+// Device buffers by column, none at first.
+struct ColumnBufs {
+  std::vector<DBufP> v;
+  bool count(uint32_t col) const { return col < v.size() && v[col]; }
+  DBufP& operator[](uint32_t col) {
+    if (col >= v.size()) v.resize(col + 1);
+    return v[col];
+  }
+  const DBufP& at(uint32_t col) const {
+    if (!count(col)) throw Error(LG_ERR_INVALID, "column without data");
+    return v[col];
+  }
+};
+
 struct Prover {
   Ctx& c;
-  Program pg;
   uint32_t num_queries;
+  ProgCache* prog = nullptr;  // compiled code of this program, kept on the context
+  std::shared_ptr<ProgCache> prog_keep;  // ... and alive while this prove lasts
+  std::shared_ptr<Layout> layout;
+  Program& pg;
+  using Group = Layout::Group;
+  using TreeL = Layout::TreeL;
   Transcript fs;
   std::vector<E6> coins;
   // Exposed values (logup totals, in step order): Montgomery E6 once read back.
@@ -62,20 +97,19 @@ struct Prover {
   std::vector<char> exposed_ready;
   DBufP exposed_d;  // 6 words per exposed value, written by k_logup_finish
   DBufP coins_dev;
-  std::vector<uint32_t> mod_order;
-  std::vector<int> fold_root, degree;
-  std::vector<bool> root_ext;
-  std::map<uint32_t, std::vector<int>> col_shifts;
+  std::vector<uint32_t>& mod_order;
+  std::vector<int>&fold_root, &degree;
+  std::vector<bool>& root_ext;
+  std::map<uint32_t, std::vector<int>>& col_shifts;
+  std::vector<TreeL>& trees;
+  std::vector<char>& ext_of;
 
   // column data on the device: lane pointer = buf + w * n
-  std::map<uint32_t, DBufP> col_buf;
+  ColumnBufs col_buf;
   DBufP witness_dev;  // host witness columns, uploaded into one buffer
   bool upload_pending = false;  // late columns of a split upload still on the side stream (await_upload)
   std::map<uint32_t, const uint32_t*> col_coef;  // committed columns: coefficient lane 0
 
-  struct Group { uint32_t module; std::vector<uint32_t> bcols, ecols; };
-  struct TreeL { bool air; int round; std::vector<Group> groups; bool setup = false; };
-  std::vector<TreeL> trees;
   std::vector<Committed> committed;
   std::vector<Digest> commitments;
   std::map<uint32_t, DBufP> chunk_coef;  // module -> chunks (d * lanes + w) * n
@@ -105,11 +139,9 @@ struct Prover {
   using DevWords = std::vector<std::pair<const uint32_t*, uint32_t>>;
   std::vector<char> fold_dev;               // fold challenges up to r0 the device computed (lg_prove)
 
-  ProgCache* prog = nullptr;  // compiled code of this program, kept on the context
-  std::shared_ptr<ProgCache> prog_keep;  // ... and alive while this prove lasts
-
   // ---- state of the phases (prove_flow.cuh), in the order they run
-  struct Poly { size_t t, g; bool ext; const uint32_t* coef; uint32_t logn; std::vector<int> shifts; };
+  // eval: its first evaluation (eval_lanes' order: per shift one, or the six lanes of an extension polynomial)
+  struct Poly { size_t t, g; bool ext; const uint32_t* coef; uint32_t logn; std::vector<int> shifts; uint32_t eval = 0; };
   size_t tree_next = 0;                     // next entry of `trees` to commit
   std::vector<char> coin_ready;             // per round: its challenge is known
   bool zeta_ready = false, alpha_ready = false;
@@ -118,6 +150,12 @@ struct Prover {
   std::vector<std::vector<std::vector<std::vector<E6>>>> cv;          // claimed values [tree][group][poly][shift]
   std::vector<uint32_t> classes;            // DEEP classes: modules with committed groups, layout order
   std::vector<DBufP> deep;                  // DEEP codeword per class (6 lanes x 4n)
+  DBufP evals_d;                            // the claimed values' lanes on the device (eval_lanes)
+  // The DEEP phase's tables, laid out while the device evaluates: everything
+  // but alpha's powers, which k_deep_weights fills in.
+  std::vector<DeepJob> deep_jobs;           // per class
+  std::vector<double> deep_bytes;
+  DBufP deep_tables;                        // DeepWeights per class and what they point to
   std::vector<DBufP> deep_den;              // per class: 1/(z_s - x) per point (k_deep_den), or empty
   bool den_pending = false;                 // k_deep_den queued on the side stream, not yet joined
   // FRI (internal/fri/fri.go:352-365,606-736)
@@ -150,14 +188,26 @@ struct Prover {
   }
   Prover(const Prover&) = delete;
   Prover& operator=(const Prover&) = delete;
-  Prover(Ctx& ctx, const uint32_t* words, size_t nwords, uint32_t q) : c(ctx), num_queries(q) {
-    pg = parse_program(words, nwords);
-    if (q == 0) throw Error(LG_ERR_INVALID, "num_queries must be positive");
-    if (q > 65535) throw Error(LG_ERR_UNSUPPORTED, "num_queries above 65535 is not supported by this build");
-    auto& L = c.programs;
+  Prover(Ctx& ctx, const uint32_t* words, size_t nwords, uint32_t q)
+      : c(ctx), num_queries(q), prog_keep(program_of(ctx, words, nwords, q)), layout(prog_keep->layout), pg(layout->pg),
+        mod_order(layout->mod_order), fold_root(layout->fold_root), degree(layout->degree),
+        root_ext(layout->root_ext), col_shifts(layout->col_shifts), trees(layout->trees), ext_of(layout->ext_of) {
+    prog = prog_keep.get();
+  }
+  // The context's entry for this descriptor, made (parsed) when it is new or
+  // when no prove of it has got through its layout yet.
+  static std::shared_ptr<ProgCache> program_of(Ctx& ctx, const uint32_t* words, size_t nwords, uint32_t q) {
+    auto& L = ctx.programs;
     auto it = std::find_if(L.begin(), L.end(), [&](const std::shared_ptr<ProgCache>& e) {
       return e->words.size() == nwords && std::equal(e->words.begin(), e->words.end(), words);
     });
+    std::shared_ptr<Layout> fresh;
+    if (it == L.end() || !(*it)->layout->ready) {
+      fresh = std::make_shared<Layout>();
+      fresh->pg = parse_program(words, nwords);
+    }
+    if (q == 0) throw Error(LG_ERR_INVALID, "num_queries must be positive");
+    if (q > 65535) throw Error(LG_ERR_UNSUPPORTED, "num_queries above 65535 is not supported by this build");
     if (it != L.end()) {
       L.splice(L.begin(), L, it);
     } else {
@@ -166,8 +216,8 @@ struct Prover {
       L.push_front(e);
       while (L.size() > Ctx::MAX_PROGRAMS) L.pop_back();
     }
-    prog_keep = L.front();
-    prog = prog_keep.get();
+    if (fresh) L.front()->layout = fresh;
+    return L.front();
   }
 
   // The bytecode of `roots` compiled in order against one lane table
@@ -243,7 +293,6 @@ struct Prover {
     if (x.op == OP_CONST) return false;
     return false;  // combined by the caller through ext_of
   }
-  std::vector<char> ext_of;  // per node
   void compute_ext() {
     ext_of.assign(pg.nodes.size(), 0);
     for (size_t i = 0; i < pg.nodes.size(); i++) {
@@ -368,6 +417,8 @@ struct Prover {
   void init_order() {
     exposed.assign(n_exposed(), e6_zero());
     exposed_ready.assign(n_exposed(), 0);
+    if (layout->ready) return;
+    mod_order.clear();
     for (uint32_t m = 0; m < pg.modules.size(); m++) mod_order.push_back(m);
     std::sort(mod_order.begin(), mod_order.end(), [&](uint32_t a, uint32_t b) { return pg.modules[a].name < pg.modules[b].name; });
   }
@@ -425,12 +476,14 @@ struct Prover {
     upload_pending = false;
     std::vector<const uint32_t*> src(pg.columns.size(), nullptr);
     size_t wi = 0, woff = 0;
+    col_buf.v.resize(pg.columns.size());
+    auto views = std::make_shared<std::vector<DBuf>>(pg.columns.size());  // the witness columns' views, one allocation
     for (uint32_t col = 0; col < pg.columns.size(); col++) {
       const Column& cl = pg.columns[col];
       size_t n = mod_n(cl.module);
       if (cl.kind == KIND_WITNESS) {
         if (cl.field != 0) throw Error(LG_ERR_UNSUPPORTED, "extension-field witness columns are not supported");
-        auto b = std::make_shared<DBuf>();
+        DBuf* b = &(*views)[col];
         b->words = n;
         b->borrowed = true;
         src[col] = witness[wi++];
@@ -441,7 +494,7 @@ struct Prover {
           b->p = witness_dev->p + woff;
           woff += n;
         }
-        col_buf[col] = b;
+        col_buf[col] = DBufP(views, b);
       } else if (cl.kind == KIND_LAGRANGE) {
         // 1 at its row: a program constant, kept on the context
         auto key = std::make_pair(pg.modules[cl.module].log_n, lagrange_row(col));
@@ -513,6 +566,9 @@ struct Prover {
   // Module order is set; folded relations, degrees, shift schedule and the
   // tree layout (no column data needed).
   void setup_layout() {
+    if (layout->ready) return;
+    if (!trees.empty() || !fold_root.empty())  // an earlier attempt threw part way
+      throw Error(LG_ERR_INVALID, "the program's layout is incomplete");
     // fold relations with coin(last round) (board/program.go:62-80)
     fold_root.assign(pg.modules.size(), -1);
     degree.assign(pg.modules.size(), NEG_INF);
@@ -598,6 +654,7 @@ struct Prover {
     if (!air.groups.empty()) trees.push_back(air);
     for (uint32_t m = 0; m < pg.modules.size(); m++)
       if (pg.modules[m].log_n > MAX_LOG_MODULE) throw Error(LG_ERR_INVALID, "module above 2^22 rows");
+    layout->ready = true;
   }
 
   // row of a Lagrange column (board/module.go:56-82: i, or N-1-i for relative rows)
@@ -1387,6 +1444,7 @@ struct Prover {
   std::vector<uint32_t> class_point_factors(uint32_t m) const;
   // k_deep_den for every class on the side stream (needs zeta in its slot)
   void launch_deep_den();
+  void prepare_deep();
   void deep_codewords();                  // internal/fri/deep.go:71-266
   Digest commit_levels();                 // fri.Prove's levels tree (internal/fri/fri.go:294-317)
   // fold round j (foldLayerExt) with the challenge at chal + 8 j, then the
