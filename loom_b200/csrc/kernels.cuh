@@ -1210,7 +1210,7 @@ struct DeepJob {
   uint32_t n_points;
   E6 z[DEEP_MAX_POINTS];
   E6 a[DEEP_MAX_POINTS];
-  const uint32_t* a_dev;  // a[0] on the device instead (null: a)
+  const uint32_t* a_dev;  // a on the device instead, six words a point (null: a)
   int logn4;            // log2 of the LDE size
   uint32_t vec;         // lanes aligned to the rows a thread takes
   const uint32_t* tw;   // w_4n^j table
@@ -1328,9 +1328,9 @@ __global__ void __launch_bounds__(DEEP_BLOCK) k_deep(const DeepJob* jobs) {
 #pragma unroll
     for (int i = 0; i < ROWS; i++) {
       acc[s][i] = jb.a[s];
-      if (ROWMAJOR && jb.a_dev)
+      if (jb.a_dev && (uint32_t)s < jb.n_points)
 #pragma unroll
-        for (int w = 0; w < 6; w++) acc[s][i].c[w] = jb.a_dev[w];
+        for (int w = 0; w < 6; w++) acc[s][i].c[w] = jb.a_dev[6 * s + w];
     }
   E6 sum[ROWS];
 #pragma unroll
@@ -1468,6 +1468,73 @@ __global__ void __launch_bounds__(256) k_deep_coefs(E6 alpha, const uint32_t* va
   E6 total;
   block_scan<true, 256>(sum, sh, total);
   if (threadIdx.x < 6) a[threadIdx.x] = total.c[threadIdx.x];
+}
+
+// The weights of a class (a block each), once alpha_DEEP is known: lane l of
+// polynomial i gets alpha^i times the basis element of its place `w` (1, u, v,
+// u v, v^2, u v^2; padding lanes nothing), and point k gets
+// a_k = sum_i alpha^i value(i, k) over the claimed values where the evaluation
+// left them (an extension polynomial's as its six lanes).
+//
+// A chain of E6 products is all that it costs, so the first powers of alpha
+// go into a table by doubling (one product a round), and a point's terms are
+// summed by a warp.
+constexpr uint32_t DEEP_NO_POLY = 0xffffffffu;
+struct DeepPlace { uint32_t poly, w; };
+struct DeepTerm { uint32_t eval, poly, ext, point; };
+struct DeepWeights {
+  DeepLane* lanes;
+  const DeepPlace* places;
+  const DeepTerm* terms;
+  uint32_t n_lanes, n_terms, n_points, n_polys;
+  uint32_t* a;
+};
+__device__ __forceinline__ E6 e6_mul_basis(E6 x, uint32_t w) {
+  if (w & 1) x = e6_mul_u(x);
+  for (uint32_t k = 0; k < w / 2; k++) x = e6_mul_v(x);
+  return x;
+}
+__global__ void __launch_bounds__(128) k_deep_weights(const DeepWeights* classes, E6 alpha, const uint32_t* evals) {
+  __shared__ E6 pw[129];
+  const DeepWeights cl = classes[blockIdx.x];
+  const uint32_t tid = threadIdx.x;
+  if (tid < 2) pw[tid] = tid ? alpha : e6_one();
+  __syncthreads();
+  for (uint32_t d = 1; d < 128 && d < cl.n_polys; d *= 2) {  // alpha^0 .. alpha^d are there
+    if (tid < d) pw[d + 1 + tid] = e6_mul(pw[d], pw[1 + tid]);
+    __syncthreads();
+  }
+  auto power = [&](uint32_t i) {
+    return i < 128 ? pw[i] : e6_mul(pw[i & 127], e6_pow(pw[128], i >> 7));
+  };
+  for (uint32_t l = tid; l < cl.n_lanes; l += 128) {
+    const DeepPlace pl = cl.places[l];
+    const E6 v = pl.poly == DEEP_NO_POLY ? e6_zero() : e6_mul_basis(power(pl.poly), pl.w);
+#pragma unroll
+    for (int w = 0; w < 6; w++) cl.lanes[l].c[w] = v.c[w];
+  }
+  for (uint32_t k = tid / 32; k < cl.n_points; k += 4) {
+    E6 sum = e6_zero();
+    for (uint32_t i = tid % 32; i < cl.n_terms; i += 32) {
+      const DeepTerm t = cl.terms[i];
+      if (t.point != k) continue;
+      E6 v = ld6(evals + 6 * (uint64_t)t.eval, 1, 0);
+      if (t.ext)
+        for (uint32_t w = 1; w < 6; w++) v = e6_add(v, e6_mul_basis(ld6(evals + 6 * ((uint64_t)t.eval + w), 1, 0), w));
+      sum = e6_add(sum, e6_mul(power(t.poly), v));
+    }
+#pragma unroll
+    for (int d = 16; d; d /= 2) {
+      E6 o;
+#pragma unroll
+      for (int w = 0; w < 6; w++) o.c[w] = __shfl_xor_sync(0xffffffffu, sum.c[w], d);
+      sum = e6_add(sum, o);
+    }
+    if (tid % 32 == 0) {
+#pragma unroll
+      for (int w = 0; w < 6; w++) cl.a[6 * k + w] = sum.c[w];
+    }
+  }
 }
 
 // ---------------------------------------------------------------- FRI
@@ -1855,6 +1922,8 @@ __global__ void k_assemble(const SectionSrc* secs, const uint32_t* map, const ui
     w = __byte_perm(v, 0, 0x0123);
   }
   out[sc.out_off + (uint64_t)k * sc.q_words + j] = w;
+  // the section's query count stands before it, as in the proof
+  if (j == 0 && k == 0) out[sc.out_off - 1] = __byte_perm(nq, 0, 0x0123);
 }
 
 }  // namespace lg

@@ -67,9 +67,10 @@ struct OpenPlan {
     for (size_t i = 0; i < n; i++) map.push_back((uint32_t)(off + i));
   }
   SectionSrc end(uint32_t nq) {
-    SectionSrc sc{start, total, (uint32_t)(map.size() - start)};
+    // a word for the query count, then the section
+    SectionSrc sc{start, total + 1, (uint32_t)(map.size() - start)};
     secs.push_back(sc);
-    total += (uint64_t)nq * sc.q_words;
+    total += 1 + (uint64_t)nq * sc.q_words;
     return sc;
   }
 
@@ -342,19 +343,24 @@ inline void Prover::claimed_values() {
           // zeta w^s with zeta read from its device slot
           auto f = factor.emplace(std::make_pair(p.logn, s), 0u);
           if (f.second) f.first->second = mont_pow(root_of_unity_mont((int)p.logn), (uint64_t)s);
+          if (s == p.shifts[0]) p.eval = (uint32_t)lanes.size();
           for (uint32_t w = 0; w < (p.ext ? 6u : 1u); w++)
             lanes.push_back(EvalLane{p.coef + ((size_t)w << p.logn), p.logn, f.first->second});
         }
   std::vector<uint32_t> dots(6 * lanes.size());
   if (!lanes.empty()) {
     auto od = eval_lanes(c, fs_slot(pg.n_rounds), lanes);
+    evals_d = od;
     // the DEEP denominators depend on zeta alone: forked after the dot
     // products, they run on the side stream while the host reads the claimed
     // values back and hashes them
     launch_deep_den();
+    prepare_deep();  // host work while the device evaluates
     uint32_t* h = c.host_staging(dots.size());
     c.d2h(h, od->p, dots.size());
     memcpy(dots.data(), h, dots.size() * 4);
+  } else {
+    prepare_deep();  // nothing opened: codewords of zeros
   }
   cv.assign(trees.size(), {});
   size_t j = 0;
@@ -364,20 +370,22 @@ inline void Prover::claimed_values() {
       for (auto& p : polys[t][g]) {
         std::vector<E6> vals;
         for (size_t si = 0; si < p.shifts.size(); si++) {
-          E6 v = e6_zero();
-          for (uint32_t w = 0; w < (p.ext ? 6u : 1u); w++, j++) {
+          auto at = [&](size_t k) {
             E6 d;
-            for (int q = 0; q < 6; q++) d.c[q] = dots[6 * j + q];
-            E6 basis = e6_zero();
-            basis.c[w] = MONT_ONE;
-            v = e6_add(v, p.ext ? e6_mul(d, basis) : d);
+            for (int q = 0; q < 6; q++) d.c[q] = dots[6 * (j + k) + q];
+            return d;
+          };
+          E6 v = at(0);
+          if (p.ext) {  // (d0 + u d1) + v ((d2 + u d3) + v (d4 + u d5))
+            auto pair = [&](size_t k) { return e6_add(at(k), e6_mul_u(at(k + 1))); };
+            v = e6_add(pair(0), e6_mul_v(e6_add(pair(2), e6_mul_v(pair(4)))));
           }
+          j += p.ext ? 6 : 1;
           vals.push_back(v);
         }
         cv[t][g].push_back(vals);
       }
   }
-  classes = deep_class_list();
 }
 
 inline std::vector<uint32_t> Prover::deep_class_list() const {
@@ -457,39 +465,34 @@ inline std::vector<E6> Prover::claimed_values_bind_order() const {
 }
 
 // ---- DEEP codewords on the LDE rows (internal/fri/deep.go:71-266)
-inline void Prover::deep_codewords() {
-  if (cv.empty()) throw Error(LG_ERR_INVALID, "the claimed values are not computed yet");
-  if (!alpha_ready) throw Error(LG_ERR_INVALID, "challenge alpha_DEEP has not been set");
-  deep.assign(classes.size(), nullptr);
-  DBufP deep_all;  // one allocation for every class's codeword
-  {
-    size_t words = 0;
-    for (uint32_t m : classes) words += 6 * (mod_n(m) << RATE_LOG);
-    deep_all = std::make_shared<DBuf>(words, c.stream);
-  }
-  size_t deep_off = 0;
-  std::vector<DeepJob> djobs;
-  std::vector<DeepLane> all_lanes;  // every class's lanes, one upload
-  std::vector<size_t> lane_off;
-  std::vector<double> dbytes;
+// Lays out every class's lanes and claimed-value terms (no challenge needed).
+inline void Prover::prepare_deep() {
+  classes = deep_class_list();
+  deep_jobs.clear();
+  deep_bytes.clear();
+  std::vector<DeepLane> lanes;  // all classes', one upload each
+  std::vector<DeepPlace> places;
+  std::vector<DeepTerm> terms;
+  std::vector<DeepWeights> weights;
+  std::vector<size_t> lane_off, term_off;
+  std::vector<uint32_t> n_polys;
+  struct Entry { DeepLane lane; DeepPlace place; };
   for (size_t ci = 0; ci < classes.size(); ci++) {
-    uint32_t m = classes[ci];
-    uint32_t logn = pg.modules[m].log_n;
-    size_t big = mod_n(m) << RATE_LOG;
-    uint32_t w_n = root_of_unity_mont((int)logn);
-    DeepJob jb{};
-    std::map<uint32_t, std::vector<DeepLane>> by_mask;  // lanes opened at the same points
+    const uint32_t m = classes[ci], logn = pg.modules[m].log_n;
+    const size_t big = mod_n(m) << RATE_LOG;
+    const uint32_t w_n = root_of_unity_mont((int)logn);
+    std::map<uint32_t, std::vector<Entry>> by_mask;  // lanes opened at the same points
+    std::vector<uint32_t> pts_w;  // the points' factors w_n^shift (first-use order, as k_deep_den)
     double row_bytes = 24.0;
-    std::vector<E6> pts;
-    std::vector<uint32_t> pts_w;  // their factors w_n^shift (first-use order, as k_deep_den)
-    E6 run = e6_one();
+    uint32_t poly = 0;
+    lane_off.push_back(lanes.size());
+    term_off.push_back(terms.size());
     for (size_t t = 0; t < trees.size(); t++)
       for (size_t g = 0; g < trees[t].groups.size(); g++) {
         if (trees[t].groups[g].module != m) continue;
         const LdeOut& l = committed[t].groups[g];
         uint32_t lane = 0;
-        for (size_t i = 0; i < polys[t][g].size(); i++) {
-          const Poly& p = polys[t][g][i];
+        for (const Poly& p : polys[t][g]) {
           const uint32_t* lane0 = l.lde->p + (size_t)lane * big;
           const uint32_t n_lanes = p.ext ? 6 : 1;
           uint32_t mask = 0;
@@ -497,51 +500,101 @@ inline void Prover::deep_codewords() {
           row_bytes += 4.0 * n_lanes;
           for (size_t si = 0; si < p.shifts.size(); si++) {
             const uint32_t f = mont_pow(w_n, (uint64_t)p.shifts[si]);
-            size_t k = 0;
+            uint32_t k = 0;
             while (k < pts_w.size() && pts_w[k] != f) k++;
-            if (k == pts.size()) {
-              if (pts.size() == DEEP_MAX_POINTS) throw Error(LG_ERR_UNSUPPORTED, "too many distinct opening points");
-              pts.push_back(e6_mul_base(zeta, f));
+            if (k == pts_w.size()) {
+              if (k == (uint32_t)DEEP_MAX_POINTS) throw Error(LG_ERR_UNSUPPORTED, "too many distinct opening points");
               pts_w.push_back(f);
-              jb.a[k] = e6_zero();
             }
-            jb.a[k] = e6_add(jb.a[k], e6_mul(run, cv[t][g][i][si]));
+            terms.push_back(DeepTerm{p.eval + (uint32_t)si * n_lanes, poly, p.ext ? 1u : 0u, k});
             mask |= 1u << k;
           }
-          E6 vrun = run;
           if (mask)  // an unopened polynomial adds nothing
-            for (uint32_t w = 0; w < n_lanes; w++) {
-              // run times the basis 1, u, v, u v, v^2, u v^2
-              if (w == 2 || w == 4) vrun = e6_mul_v(vrun);
-              const E6 scale = w & 1 ? e6_mul_u(vrun) : vrun;
-              DeepLane dl{lane0 + (size_t)w * big, {}, mask, 0};
-              memcpy(dl.c, scale.c, 24);
-              by_mask[mask].push_back(dl);
-            }
-          run = e6_mul(run, alpha);
+            for (uint32_t w = 0; w < n_lanes; w++)
+              by_mask[mask].push_back(Entry{DeepLane{lane0 + (size_t)w * big, {}, mask, 0}, DeepPlace{poly, w}});
+          poly++;
         }
       }
-    for (size_t k = 0; k < pts.size(); k++) jb.z[k] = pts[k];
-    jb.n_points = (uint32_t)pts.size();
-    lane_off.push_back(all_lanes.size());
+    n_polys.push_back(poly);
     for (auto& kv : by_mask) {  // whole quads of one mask
       auto& v = kv.second;
-      v.resize((v.size() + 3) / 4 * 4, DeepLane{v[0].p, {0, 0, 0, 0, 0, 0}, kv.first, 0});
-      all_lanes.insert(all_lanes.end(), v.begin(), v.end());
+      v.resize((v.size() + 3) / 4 * 4, Entry{v[0].lane, DeepPlace{DEEP_NO_POLY, 0}});
+      for (auto& e : v) {
+        lanes.push_back(e.lane);
+        places.push_back(e.place);
+      }
     }
-    jb.n_lanes = (uint32_t)(all_lanes.size() - lane_off.back());
+    DeepJob jb{};
+    jb.n_points = (uint32_t)pts_w.size();
+    for (size_t k = 0; k < pts_w.size(); k++) jb.z[k] = e6_base(pts_w[k]);  // times zeta, in deep_codewords
+    jb.n_lanes = (uint32_t)(lanes.size() - lane_off.back());
     jb.vec = 1;
     jb.logn4 = (int)logn + RATE_LOG;
     jb.tw = c.twiddles(jb.logn4);
+    deep_jobs.push_back(jb);
+    deep_bytes.push_back(row_bytes * big);
+  }
+  // one buffer: the weights' records, lanes, places and terms, then the points'
+  // sums (written on the device)
+  static_assert(sizeof(DeepWeights) % 8 == 0 && sizeof(DeepLane) % 8 == 0 && sizeof(DeepPlace) % 8 == 0 &&
+                sizeof(DeepTerm) % 8 == 0, "tables packed one after another");
+  const size_t lanes_at = classes.size() * sizeof(DeepWeights);
+  const size_t places_at = lanes_at + lanes.size() * sizeof(DeepLane);
+  const size_t terms_at = places_at + places.size() * sizeof(DeepPlace);
+  const size_t sums_at = terms_at + terms.size() * sizeof(DeepTerm);
+  const size_t sum_words = 6 * (size_t)DEEP_MAX_POINTS * classes.size();
+  deep_tables = std::make_shared<DBuf>(std::max<size_t>(1, sums_at / 4 + sum_words), c.stream);
+  uint8_t* base = (uint8_t*)deep_tables->p;
+  for (size_t ci = 0; ci < classes.size(); ci++) {
+    const size_t next = ci + 1 < classes.size() ? term_off[ci + 1] : terms.size();
+    DeepWeights w{};
+    w.lanes = (DeepLane*)(base + lanes_at) + lane_off[ci];
+    w.places = (const DeepPlace*)(base + places_at) + lane_off[ci];
+    w.terms = (const DeepTerm*)(base + terms_at) + term_off[ci];
+    w.n_lanes = deep_jobs[ci].n_lanes;
+    w.n_terms = (uint32_t)(next - term_off[ci]);
+    w.n_points = deep_jobs[ci].n_points;
+    w.n_polys = n_polys[ci];
+    w.a = (uint32_t*)(base + sums_at) + 6 * DEEP_MAX_POINTS * ci;
+    weights.push_back(w);
+    deep_jobs[ci].lanes = w.lanes;
+    deep_jobs[ci].a_dev = w.a;
+  }
+  std::vector<uint8_t> host(sums_at);
+  auto put = [&](size_t at, const auto& v) {
+    if (!v.empty()) memcpy(host.data() + at, v.data(), v.size() * sizeof(v[0]));
+  };
+  put(0, weights);
+  put(lanes_at, lanes);
+  put(places_at, places);
+  put(terms_at, terms);
+  if (sums_at) c.h2d(deep_tables->p, host.data(), sums_at);
+}
+
+inline void Prover::deep_codewords() {
+  if (cv.empty()) throw Error(LG_ERR_INVALID, "the claimed values are not computed yet");
+  if (!alpha_ready) throw Error(LG_ERR_INVALID, "challenge alpha_DEEP has not been set");
+  std::vector<DeepJob> djobs = deep_jobs;
+  const std::vector<double>& dbytes = deep_bytes;
+  size_t words = 0, deep_off = 0;
+  for (uint32_t m : classes) words += 6 * (mod_n(m) << RATE_LOG);
+  auto deep_all = std::make_shared<DBuf>(words, c.stream);  // one allocation for every class's codeword
+  deep.assign(classes.size(), nullptr);
+  for (size_t ci = 0; ci < djobs.size(); ci++) {
+    const size_t big = mod_n(classes[ci]) << RATE_LOG;
     deep[ci] = dbuf_slice(deep_all, deep_off, 6 * big);
     deep_off += 6 * big;
-    jb.out = deep[ci]->p;
-    if (den_pending && ci < deep_den.size() && deep_den[ci]) jb.den = deep_den[ci]->p;
-    djobs.push_back(jb);
-    dbytes.push_back(row_bytes * big);
+    djobs[ci].out = deep[ci]->p;
+    for (uint32_t k = 0; k < djobs[ci].n_points; k++) djobs[ci].z[k] = e6_mul_base(zeta, djobs[ci].z[k].c[0]);
+    if (den_pending && ci < deep_den.size() && deep_den[ci]) djobs[ci].den = deep_den[ci]->p;
   }
-  auto lanes_d = upload_vec(c, all_lanes);
-  for (size_t i = 0; i < djobs.size(); i++) djobs[i].lanes = (const DeepLane*)lanes_d->p + lane_off[i];
+  if (!djobs.empty()) {
+    c.timed("deep", 0, 0, [&] {
+      k_deep_weights<<<(unsigned)djobs.size(), 128, 0, c.stream>>>((const DeepWeights*)deep_tables->p, alpha,
+                                                                evals_d ? evals_d->p : nullptr);
+      LG_LAUNCH();
+    });
+  }
   if (den_pending) {  // join the side stream's denominators
     LG_CK(cudaStreamWaitEvent(c.stream, c.join_ev, 0));
     den_pending = false;
@@ -857,11 +910,28 @@ inline size_t Prover::open_and_encode(const std::vector<uint32_t>& pos, uint8_t*
   }
   Writer W(c.proof_buf, out, out_cap);
   if (pinned) {
+    // sections that follow one another here and in the proof, the query count
+    // before each included (the device wrote the same word), go in one copy
+    uint8_t* run_dst = nullptr;
+    uint64_t run_off = 0;
+    size_t run_bytes = 0;
+    auto flush = [&] {
+      if (run_bytes) LG_CK(cudaMemcpyAsync(run_dst, asm_d->p + run_off, run_bytes, cudaMemcpyDeviceToHost, c.stream));
+      run_bytes = 0;
+    };
     emit(W, [&](Writer& Wr, const SectionSrc& sc) {
       const size_t n = sec_bytes(sc);
       uint8_t* dst = Wr.claim(n);
-      LG_CK(cudaMemcpyAsync(dst, asm_d->p + sc.out_off, n, cudaMemcpyDeviceToHost, c.stream));
+      if (run_bytes && dst == run_dst + run_bytes + 4 && sc.out_off == run_off + run_bytes / 4 + 1) {
+        run_bytes += 4 + n;
+      } else {
+        flush();
+        run_dst = dst;
+        run_off = sc.out_off;
+        run_bytes = n;
+      }
     });
+    flush();
   } else {
     uint32_t* A = c.host_staging(OP.total);
     c.d2h(A, asm_d->p, OP.total);
