@@ -1311,7 +1311,7 @@ template <int ROWS> __device__ __forceinline__ void deep_inverses(const E6& z, c
 // one point, the denominators computed here.  NP: points held in registers
 // (at least the job's).
 // What bounds it: the integer-multiply pipe (6 wide products per lane and row).
-// 48 lanes of 2^20 rows on B200: 150 us a call (349 us lane by lane, with the
+// 48 lanes of 2^20 rows on B200: 138 us a call (349 us lane by lane, with the
 // points' sums in local memory and a transposing pass after it).
 constexpr int DEEP_BLOCK = 128, DEEP_STAGE = 64;
 template <int NP, int ROWS, bool ROWMAJOR>
@@ -1584,7 +1584,7 @@ __global__ void k_fold(const uint32_t* layer, uint64_t n, const uint32_t* alpha_
 // rather than a scattered read of a table as long as the layer.  VEC: 16- and
 // 8-byte accesses (the caller's rows aligned to 16 bytes).
 // What bounds it: HBM and the integer pipes about equally (72 B and 30
-// products per output row).  2^22 rows on B200: 54 us a call, 0.42 of the
+// products per output row).  2^22 rows on B200: 48 us a call, 0.48 of the
 // measured HBM rate (257 us with a copy in, a transpose, the fold, a transpose
 // back and a copy out).
 constexpr int FOLD_SPLIT = 11;

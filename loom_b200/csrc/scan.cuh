@@ -99,7 +99,8 @@ inline uint32_t gp_tile(uint64_t n) { return n <= 1u << 16 ? GP_TILE_S : n <= 1u
 // What bounds it: the integer-multiply pipe (about five E6 products a row)
 // and, for few tiles, the dependent products of the scan and the inversion.
 // 512 threads an SM, 128 registers each: with both operands of every row held
-// (210 registers) 1,000,003 rows took 162 us, so 127 (start to end).
+// (210 registers) 1,000,003 rows took 162 us and not 127 (start to end; 98 with
+// the extension products of one reduction per coefficient).
 template <int T, int R, bool VEC, bool RATIO>
 __global__ void __launch_bounds__(T, 512 / T) k_rows_scan(const uint32_t* num, const uint32_t* den, uint64_t n,
                                                           uint32_t* x, uint32_t* totals) {
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(T, 512 / T) k_rows_scan(const uint32_t* num, c
   const E6 pre = block_scan<false, T>(acc, sh, total);
 #pragma unroll
   for (int i = 0; i < R; i++)
-    if (base + i < n) st_row<VEC>(x, base + i, e6_mul(pre, v[i]));
+    if (base + i < n) st_row<VEC>(x, base + i, e6_mul(v[i], pre));
   if (threadIdx.x < 6) totals[6 * (uint64_t)blockIdx.x + threadIdx.x] = total.c[threadIdx.x];
 }
 
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(T, 512 / T) k_rows_apply(uint32_t* x, uint64_t
   }
 #pragma unroll
   for (int i = 0; i < R; i++)
-    if (first + i * T < n) st_row<VEC>(x, first + i * T, e6_mul(p, v[i]));
+    if (first + i * T < n) st_row<VEC>(x, first + i * T, e6_mul(v[i], p));
 }
 
 // Exclusive prefix products of nt tile totals, one block of T threads.
