@@ -461,8 +461,12 @@ struct Ctx {
     uint32_t quotient_jit = 1;          // constraint bytecode (quotient, grand-product ratios) as compiled kernels (0: interpreter)
     uint32_t upload_split = 1;          // host witness: round 0's columns first, the rest on the side stream while
                                         // round 0 runs (0: every column before the prove starts)
-    uint32_t fri_tail_leaves = 0;       // FRI rounds whose layer tree has at most this many leaves: one block (0: none;
-                                        // 512 measured 14.09 ms against 13.65 ms per 40 x 2^14 prove)
+    // FRI rounds whose layer tree has at most this many leaves: one block (0:
+    // none).  Proves on B200, us, for 0 / 8 / 16 / 32 / 64 / 128 / 256: the
+    // small circuit 842 / 826 / 811 / 795 / 794 / 792 / 794; 40 modules of
+    // 2^14 rows 8675 / 8657 / 8650 / 8633 / 8624 / 8624 / 8641.  Above 64 a
+    // tree's leaves no longer fit a block's warps at once.
+    uint32_t fri_tail_leaves = 64;
   } tune;
 };
 

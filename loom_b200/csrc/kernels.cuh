@@ -546,7 +546,7 @@ __global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, con
   P2Lane L;
   L.init(keys);
   const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5, per = warps * P2_GROUPS_PER_WARP;
-  const uint32_t nb = gridDim.x, b = blockIdx.x, slot = warp * P2_GROUPS_PER_WARP + (uint32_t)L.base / 6;
+  const uint32_t nb = gridDim.x, b = blockIdx.x, first = warp * P2_GROUPS_PER_WARP, group = (uint32_t)L.base / 6;
   auto fold = [&](uint32_t w) {
     uint32_t cnt = 0;
     for (uint32_t t = 0; t < n_inj && cnt < 64; t++)
@@ -557,8 +557,8 @@ __global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, con
     __syncthreads();
     const uint32_t share = w / nb;
     if (cnt)
-      for (uint32_t j0 = 0; j0 < share; j0 += per) {
-        const uint32_t jl = j0 + slot, j = b * share + jl;
+      for (uint32_t j0 = first; j0 < share; j0 += per) {
+        const uint32_t jl = j0 + group, j = b * share + jl;
         merkle_chain(nodes, (uint64_t)w + j, j, chain, cnt, L, keys, L.lane < 30 && jl < share);
       }
     __syncthreads();
@@ -566,8 +566,8 @@ __global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, con
   if (fold_first) fold(top);
   for (uint32_t w = top >> 1; w >= nb; w >>= 1) {
     const uint32_t share = w / nb;
-    for (uint32_t i0 = 0; i0 < share; i0 += per) {
-      const uint32_t il = i0 + slot;
+    for (uint32_t i0 = first; i0 < share; i0 += per) {  // a warp without a node skips the level
+      const uint32_t il = i0 + group;
       merkle_node(nodes, (uint64_t)w + b * share + il, L, keys, L.lane < 30 && il < share);
     }
     __syncthreads();
@@ -1642,11 +1642,13 @@ __global__ void __launch_bounds__(256) k_fold_rows(const uint32_t* layer, FoldAr
 // with challenge j (as k_fold), the levels that enter at j + 1 (as
 // k_axpy_e6), then, unless j is the last round, layer j + 1's commitment —
 // pair leaves (one permutation each, as k_hash_leaves), the tree level by
-// level — and challenge j + 1 from its root (as k_fs_challenge).  These
-// layers are small (at most a few thousand leaves), so their launches were
-// latency bound: one block runs them back to back with barriers instead,
-// every value written where the per-round launches write it.  Six lanes per
-// permutation, five permutations per warp.
+// level — and challenge j + 1 from its root (as k_fs_challenge).  Every value
+// is written where the per-round launches write it.  Six lanes per
+// permutation, five permutations per warp; a warp without a permutation
+// leaves the schedulers to the others.
+// What bounds it: the latency of 3 + log2(leaves) dependent permutations a
+// round (2.7 us each); three launches a round add their starts to that.
+constexpr int FRI_TAIL_BLOCK = 512;
 struct FriRound {
   const uint32_t* cur;     // layer j: 6 lanes of n words (bit-reversed rows)
   uint32_t* next;          // layer j + 1: 6 lanes of n / 2 words
@@ -1657,16 +1659,16 @@ struct FriRound {
   uint32_t pre_off, pre_len;      // challenge j + 1's name elements in `pre`
   uint32_t term_first, term_count;  // levels added to layer j + 1
 };
-__global__ void __launch_bounds__(1024) k_fri_tail(const FriRound* rounds, uint32_t n_rounds, uint32_t j0,
+__global__ void __launch_bounds__(FRI_TAIL_BLOCK) k_fri_tail(const FriRound* rounds, uint32_t n_rounds, uint32_t j0,
                                                    const AxpyTerm* terms, const uint32_t* pre, uint32_t* chal,
                                                    uint32_t inv2) {
-  __shared__ __align__(16) uint32_t keys[p2c_smem_words(32)];
+  __shared__ __align__(16) uint32_t keys[p2c_smem_words(FRI_TAIL_BLOCK / 32)];
   __shared__ uint32_t msg[64];
   p2_load_full_keys(keys);  // ends with a barrier
   P2Lane L;
   L.init(keys);
-  const uint32_t warps = blockDim.x >> 5, per = warps * P2_GROUPS_PER_WARP;
-  const uint32_t slot = (threadIdx.x >> 5) * P2_GROUPS_PER_WARP + (uint32_t)L.base / 6;
+  const uint32_t per = (blockDim.x >> 5) * P2_GROUPS_PER_WARP;
+  const uint32_t first = (threadIdx.x >> 5) * P2_GROUPS_PER_WARP, group = (uint32_t)L.base / 6;
   for (uint32_t r = 0; r < n_rounds; r++) {
     const FriRound R = rounds[r];
     const uint32_t j = j0 + r;
@@ -1706,8 +1708,8 @@ __global__ void __launch_bounds__(1024) k_fri_tail(const FriRound* rounds, uint3
       g.n_leaves = nl;
       g.out = R.nodes + (size_t)8 * nl;
       const uint32_t h0 = to_mont(LEAF_TAG), h1 = to_mont(0), h2 = to_mont(2);
-      for (uint32_t k0 = 0; k0 < nl; k0 += per) {
-        const uint32_t k = k0 + slot;
+      for (uint32_t k0 = first; k0 < nl; k0 += per) {
+        const uint32_t k = k0 + group;
         const bool active = L.lane < 30 && k < nl;
         uint32_t x[4] = {0, 0, 0, 0};
         if (active && L.idx < 4) {
@@ -1727,8 +1729,8 @@ __global__ void __launch_bounds__(1024) k_fri_tail(const FriRound* rounds, uint3
     }
     __syncthreads();
     for (uint32_t w = nl >> 1; w >= 1; w >>= 1) {
-      for (uint32_t i0 = 0; i0 < w; i0 += per) {
-        const uint32_t i = i0 + slot;
+      for (uint32_t i0 = first; i0 < w; i0 += per) {
+        const uint32_t i = i0 + group;
         merkle_node(R.nodes, (uint64_t)w + i, L, keys, L.lane < 30 && i < w);
       }
       __syncthreads();

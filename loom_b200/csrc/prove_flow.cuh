@@ -766,7 +766,10 @@ inline void Prover::fri_tail(int j0, const DBufP& pre_d, const std::vector<uint3
   double perms = 0;
   for (auto& R : rr) if (R.nodes) perms += 2.0 * (1u << R.log_leaves);
   c.timed("fri_tail", 0, perms, [&] {
-    k_fri_tail<<<1, 1024, 0, c.stream>>>((const FriRound*)rd->p, (uint32_t)rr.size(), (uint32_t)j0,
+    // a group of lanes for each leaf of the first tree, as far as a block goes
+    const uint32_t nl = rr[0].nodes ? 1u << rr[0].log_leaves : 1;
+    const uint32_t warps = std::min<uint32_t>(FRI_TAIL_BLOCK / 32, (nl + P2_GROUPS_PER_WARP - 1) / P2_GROUPS_PER_WARP);
+    k_fri_tail<<<1, 32 * warps, 0, c.stream>>>((const FriRound*)rd->p, (uint32_t)rr.size(), (uint32_t)j0,
                                           (const AxpyTerm*)td->p, pre_d->p, chal->p, inv(to_mont(2)));
     LG_LAUNCH();
   });
