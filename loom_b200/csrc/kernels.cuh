@@ -460,10 +460,14 @@ __device__ __forceinline__ void merkle_node(uint32_t* nodes, uint64_t id, const 
 __device__ __forceinline__ void merkle_chain(uint32_t* nodes, uint64_t id, uint32_t j, const uint32_t* const* inj,
                                              uint32_t n_inj, const P2Lane& L, uint32_t* keys, bool active) {
   if (n_inj == 0) return;
-  uint32_t x[4] = {0, 0, 0, 0};
+  uint32_t x[4] = {0, 0, 0, 0}, next[4] = {0, 0, 0, 0};
   p2c_load_slot(x, L, 1, nodes + id * 8, active);
+  p2c_load_slot(next, L, 2, inj[0] + (uint64_t)j * 8, active);
   for (uint32_t t = 0; t < n_inj; t++) {
-    p2c_load_slot(x, L, 2, inj[t] + (uint64_t)j * 8, active);
+    if ((L.idx >> 1) == 2)
+#pragma unroll
+      for (int i = 0; i < 4; i++) x[i] = next[i];
+    if (t + 1 < n_inj) p2c_load_slot(next, L, 2, inj[t + 1] + (uint64_t)j * 8, active);  // beside the permutation
     p2c_compress(x, L, keys);
     if (t + 1 < n_inj) p2c_digest_to_left(x, L);
   }
@@ -515,10 +519,13 @@ __global__ void __launch_bounds__(P2_MAX_BLOCK, 2) k_merkle_inject1(uint32_t* no
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= start) return;
   uint32_t* nd = nodes + ((uint64_t)start + j) * 8;
-  uint32_t l[8], r[8];
+  uint32_t l[8], r[8], next[8];
   ld_digest(nd, l);
+  ld_digest(inj[0] + (uint64_t)j * 8, next);
   for (uint32_t t = 0; t < n_inj; t++) {
-    ld_digest(inj[t] + (uint64_t)j * 8, r);
+#pragma unroll
+    for (int w = 0; w < 8; w++) r[w] = next[w];
+    if (t + 1 < n_inj) ld_digest(inj[t + 1] + (uint64_t)j * 8, next);  // beside the permutation
     p2_compress(to_mont(NODE_TAG), l, r, l);
   }
   st_digest(nd, l);
