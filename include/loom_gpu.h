@@ -125,14 +125,16 @@ int lg_ctx_set_leaf_mapping(lg_ctx* ctx, int lanes_per_permutation);
  *   "merkle_subtree"      above that, one launch builds the levels over
  *                         this many nodes per block (power of two, 2..1024;
  *                         0: a launch per level)
- *   "inject_block", "leaf_block"  threads per block (power of two, 32..1024)
+ *   "inject_block", "leaf_block"  threads per block (power of two, 32..1024;
+ *                         above 256 counts as 256)
  *   "lde_split"           1: the LDE of 2^4..2^14 rows as an inverse launch
  *                         plus one block per (lane, coset); 0: one block per
  *                         lane for all of it
  *   "lde_fwd_threads"     threads per coset block (256, 512 or 1024)
  *   "fri_tail_leaves"     the FRI rounds whose layer tree has at most this many
  *                         leaves run in one block, back to back (power of two,
- *                         2..65536; 0: a launch per step of every round)
+ *                         2..65536; 0: a launch per step of every round;
+ *                         default 64)
  *   "quotient_jit"        1: the constraint bytecode of each module's quotient
  *                         and of each grand product's ratio is compiled to a
  *                         kernel of its own at run time (NVRTC, cached per
