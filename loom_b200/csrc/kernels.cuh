@@ -1216,8 +1216,7 @@ struct DeepJob {
   uint32_t n_lanes;     // a multiple of four
   uint32_t n_points;
   E6 z[DEEP_MAX_POINTS];
-  E6 a[DEEP_MAX_POINTS];
-  const uint32_t* a_dev;  // a on the device instead, six words a point (null: a)
+  const uint32_t* a;    // the points' weighted values, six words each (device)
   int logn4;            // log2 of the LDE size
   uint32_t vec;         // lanes aligned to the rows a thread takes
   const uint32_t* tw;   // w_4n^j table
@@ -1334,10 +1333,10 @@ __global__ void __launch_bounds__(DEEP_BLOCK) k_deep(const DeepJob* jobs) {
   for (int s = 0; s < NP; s++)
 #pragma unroll
     for (int i = 0; i < ROWS; i++) {
-      acc[s][i] = jb.a[s];
-      if (jb.a_dev && (uint32_t)s < jb.n_points)
+      acc[s][i] = e6_zero();
+      if ((uint32_t)s < jb.n_points)
 #pragma unroll
-        for (int w = 0; w < 6; w++) acc[s][i].c[w] = jb.a_dev[6 * s + w];
+        for (int w = 0; w < 6; w++) acc[s][i].c[w] = jb.a[6 * s + w];
     }
   E6 sum[ROWS];
 #pragma unroll

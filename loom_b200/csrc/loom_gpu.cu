@@ -869,7 +869,7 @@ int lg_deep_quotient(lg_ctx* ctx, const uint32_t* lde, uint32_t n_cols, uint64_t
     DeepJob jb{};
     jb.n_points = 1;
     jb.z[0] = zz;
-    jb.a_dev = sum->p;
+    jb.a = sum->p;
     jb.lanes = (const DeepLane*)ld->p;
     jb.n_lanes = (uint32_t)lanes.size();
     jb.logn4 = logr;

@@ -558,7 +558,7 @@ inline void Prover::prepare_deep() {
     w.a = (uint32_t*)(base + sums_at) + 6 * DEEP_MAX_POINTS * ci;
     weights.push_back(w);
     deep_jobs[ci].lanes = w.lanes;
-    deep_jobs[ci].a_dev = w.a;
+    deep_jobs[ci].a = w.a;
   }
   std::vector<uint8_t> host(sums_at);
   auto put = [&](size_t at, const auto& v) {
