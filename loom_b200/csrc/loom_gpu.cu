@@ -28,6 +28,17 @@ __global__ void __launch_bounds__(256) k_rows_to_lanes(const RowsCol* cols) {
   st6(col.lanes, col.n, i, v);
 }
 
+// A call that fails part way has work queued that reads and writes the
+// caller's buffers: it ends before the call returns, and the error it left
+// behind is not the next call's.
+int failed(lg_ctx* ctx, int code, const char* what) {
+  ctx->c.err = what;
+  if (ctx->c.stream) cudaStreamSynchronize(ctx->c.stream);
+  if (ctx->c.side) cudaStreamSynchronize(ctx->c.side);
+  cudaGetLastError();
+  return code;
+}
+
 template <class F> int guarded(lg_ctx* ctx, F f) {
   if (!ctx) return LG_ERR_INVALID;
   try {
@@ -42,11 +53,9 @@ template <class F> int guarded(lg_ctx* ctx, F f) {
     f();
     return LG_OK;
   } catch (Error& e) {
-    ctx->c.err = e.what();
-    return e.code;
+    return failed(ctx, e.code, e.what());
   } catch (std::exception& e) {
-    ctx->c.err = e.what();
-    return LG_ERR_INVALID;
+    return failed(ctx, LG_ERR_INVALID, e.what());
   }
 }
 
