@@ -61,7 +61,10 @@ inline void check_ntt_size(int logn) {
 }
 
 // Runs four-step transforms of 2^logn points (logn > SMEM_NTT_MAX_LOG), all
-// jobs of one direction, in chunks whose scratch stays below 256 MiB.
+// jobs of one direction, in chunks of 2^26 words (256 MiB).  Jobs without a
+// scratch of their own take turns in one buffer of a chunk.  Everything is
+// allocated before the first launch: a call that the memory budget refuses has
+// written nothing.
 inline void big_ntt(Ctx& c, std::vector<BigNtt> jobs, int logn, bool inverse, const char* tag, double bytes_per_job) {
   if (jobs.empty()) return;
   const int logr = logn / 2, logc = logn - logr;
@@ -73,36 +76,36 @@ inline void big_ntt(Ctx& c, std::vector<BigNtt> jobs, int logn, bool inverse, co
   // for the coset shifts, w_{4n}
   const uint2* tw_n = c.split_powers(logn);
   const uint2* t2s = c.split_powers(logn + RATE_LOG);
-  for (auto& j : jobs) {
+  const size_t per = std::max<size_t>(1, ((size_t)1 << 26) / n);
+  DBufP scratch = jobs[0].scratch ? DBufP() : std::make_shared<DBuf>(std::min(per, jobs.size()) * n, c.stream);
+  for (size_t i = 0; i < jobs.size(); i++) {
+    BigNtt& j = jobs[i];
     if (j.t2 && j.m2_mask != (uint32_t)((n << RATE_LOG) - 1))
       throw Error(LG_ERR_INVALID, "four-step coset table of another size");
     j.c0c = from_mont(j.c0);
     j.c0s = shoup(j.c0c);
+    if (scratch) j.scratch = scratch->p + i % per * n;
   }
-  // scratch chunks of 2^26 words at most (256 MiB)
-  const size_t per = std::max<size_t>(1, ((size_t)1 << 26) / n);
+  auto jd = upload_vec(c, jobs);
   const size_t smem_a = tile_words(logc) * 4, smem_b = tile_words(logr) * 4;
   const unsigned thr_a = (unsigned)std::min<size_t>(512, (size_t)1 << logc);
   const unsigned thr_b = (unsigned)std::min<size_t>(512, (size_t)1 << logr);
   for (size_t first = 0; first < jobs.size(); first += per) {
-    size_t cnt = std::min(per, jobs.size() - first);
-    auto scratch = std::make_shared<DBuf>(cnt * n, c.stream);
-    std::vector<BigNtt> v(jobs.begin() + first, jobs.begin() + first + cnt);
-    for (size_t i = 0; i < cnt; i++) v[i].scratch = scratch->p + i * n;
-    auto jd = upload_vec(c, v);
+    const size_t cnt = std::min(per, jobs.size() - first);
+    const BigNtt* j = (const BigNtt*)jd->p + first;
     c.timed(tag, bytes_per_job * cnt, 0, [&] {
       with_tile_size(logc, [&](auto LC) {
         constexpr int C_ = decltype(LC)::value;
         allow_smem(k_big_pass_a<C_>, smem_a);
         k_big_pass_a<C_><<<dim3((1u << logr) / BIG_TILE, (unsigned)cnt), thr_a, smem_a, c.stream>>>(
-            (const BigNtt*)jd->p, logn, logr, inverse ? 1 : 0, tw_n, t2s, tw_c);
+            j, logn, logr, inverse ? 1 : 0, tw_n, t2s, tw_c);
         LG_LAUNCH();
       });
       with_tile_size(logr, [&](auto LR) {
         constexpr int R_ = decltype(LR)::value;
         allow_smem(k_big_pass_b<R_>, smem_b);
         k_big_pass_b<R_><<<dim3((1u << logc) / BIG_TILE, (unsigned)cnt), thr_b, smem_b, c.stream>>>(
-            (const BigNtt*)jd->p, logc, inverse ? 1 : 0, tw_r);
+            j, logc, inverse ? 1 : 0, tw_r);
         LG_LAUNCH();
       });
     });
@@ -111,21 +114,25 @@ inline void big_ntt(Ctx& c, std::vector<BigNtt> jobs, int logn, bool inverse, co
 
 // Coset transforms of 2^logn points (logn > SMEM_NTT_MAX_LOG) by the forward
 // tree, coefficients to bit-reversed evaluations.  Jobs go in chunks whose
-// output stays in L2 between the two passes (FWD_CHUNK words).
+// output stays in L2 between the two passes (FWD_CHUNK words).  plan_fwd
+// allocates, big_fwd launches.
 constexpr size_t FWD_CHUNK = (size_t)1 << 24;
-inline void big_fwd(Ctx& c, const std::vector<FwdJob>& jobs, int logn, const char* tag, double bytes_per_job) {
-  if (jobs.empty()) return;
-  const int logr = logn / 2, logc = logn - logr;
-  if (logr < 7 || logc > 11) throw Error(LG_ERR_UNSUPPORTED, "forward transform size out of range");
+struct FwdPlan { DBufP jobs; size_t count; int logn; const uint2* tau; };
+inline FwdPlan plan_fwd(Ctx& c, const std::vector<FwdJob>& jobs, int logn) {
+  if (logn / 2 < 7 || logn - logn / 2 > 11) throw Error(LG_ERR_UNSUPPORTED, "forward transform size out of range");
   const uint2* tau = c.tree_twiddles(logn + RATE_LOG - 1);
-  auto jd = upload_vec(c, jobs);
+  return {upload_vec(c, jobs), jobs.size(), logn, tau};
+}
+inline void big_fwd(Ctx& c, const FwdPlan& plan, const char* tag, double bytes_per_job) {
+  const int logr = plan.logn / 2, logc = plan.logn - logr;
+  const uint2* tau = plan.tau;
   const size_t smem = tile_words(logc) * 4;
   const unsigned thr = (unsigned)std::min<size_t>(512, (size_t)1 << logc);
-  const size_t per = std::min<size_t>(65535, std::max<size_t>(1, FWD_CHUNK >> logn));
-  c.timed(tag, bytes_per_job * jobs.size(), 0, [&] {
-    for (size_t first = 0; first < jobs.size(); first += per) {
-      const unsigned cnt = (unsigned)std::min(per, jobs.size() - first);
-      const FwdJob* j = (const FwdJob*)jd->p + first;
+  const size_t per = std::min<size_t>(65535, std::max<size_t>(1, FWD_CHUNK >> plan.logn));
+  c.timed(tag, bytes_per_job * plan.count, 0, [&] {
+    for (size_t first = 0; first < plan.count; first += per) {
+      const unsigned cnt = (unsigned)std::min(per, plan.count - first);
+      const FwdJob* j = (const FwdJob*)plan.jobs->p + first;
       with_tile_size(logc, [&](auto LC) {
         constexpr int C_ = decltype(LC)::value;
         allow_smem(k_fwd_cols<C_>, smem);
@@ -172,16 +179,18 @@ inline void launch_lde(Ctx& c, const std::vector<LdeLane>& lanes, uint32_t log_n
       } else {
         uint32_t* dst = lanes[i].coef ? lanes[i].coef : tmp->p + i * n;
         inv_jobs.push_back(big_job(lanes[i].src, dst, inv(to_mont((uint32_t)n)), false));
-        inv_jobs.back().coset0 = lanes[i].out;  // <w_n> itself: the values in bit-reversed order
+        inv_jobs.back().coset0 = lanes[i].out;       // <w_n> itself: the values in bit-reversed order
+        inv_jobs.back().scratch = lanes[i].out + n;  // coset 1, not written before the forward transforms
         coef[i] = dst;
       }
     }
-    big_ntt(c, inv_jobs, (int)log_n, true, "lde", 8.0 * n);
     const uint32_t a0 = from_coeffs ? 0 : 1;
     for (size_t i = 0; i < lanes.size(); i++)
       for (uint32_t a = a0; a < (1u << RATE_LOG); a++)
         fwd_jobs.push_back(FwdJob{coef[i], lanes[i].out + (size_t)a * n, a});
-    big_fwd(c, fwd_jobs, (int)log_n, "lde", 20.0 * n / (1 << RATE_LOG));
+    const FwdPlan fwd = plan_fwd(c, fwd_jobs, (int)log_n);  // allocated before the first transform
+    big_ntt(c, inv_jobs, (int)log_n, true, "lde", 8.0 * n);
+    big_fwd(c, fwd, "lde", 20.0 * n / (1 << RATE_LOG));
     return;
   }
   const uint32_t* twn = c.ntt_twiddles((int)log_n);

@@ -61,3 +61,30 @@ def test_a_failed_call_leaves_nothing_running():
     small = F.to_mont(np.arange(1, 17, dtype=np.uint32))
     assert np.array_equal(ctx.rs_encode(small)[0], oracle.rs_encode(small, 64))
     ctx.close()
+
+
+@pytest.mark.parametrize("logn,cols", [(12, 40), (15, 3), (17, 40), (20, 24)])
+def test_an_encoding_that_does_not_fit_leaves_its_output_alone(logn, cols):
+    """Device columns are encoded into the caller's buffer; whatever the budget
+    refuses, it refuses before the first word is written."""
+    import torch
+    n = 1 << logn
+    src, dst = dev(cols * n, 2), torch.empty(4 * cols * n, dtype=torch.int32, device="cuda:0")
+    roomy = Context(0)
+    encode(roomy, src, n, cols, dst)
+    want, peak = dst.clone(), roomy.mem_usage()[1]
+    roomy.close()
+    refused = 0
+    for part in range(1, 17):
+        ctx = Context(0, hbm_budget=max(1, peak * part // 16))
+        dst.fill_(-1)
+        torch.cuda.synchronize()
+        try:
+            encode(ctx, src, n, cols, dst)
+            assert torch.equal(dst, want)
+        except LoomError as e:
+            assert e.code == _lib.LG_ERR_OOM
+            assert bool((dst == -1).all()), f"refused at {part}/16 of {peak} bytes"
+            refused += 1
+        ctx.close()
+    assert 0 < refused < 16
