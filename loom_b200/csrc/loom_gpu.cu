@@ -349,25 +349,12 @@ std::vector<GroupSpec> batch_groups(Ctx& c, uint32_t n_groups, const uint64_t* r
     keep.push_back(std::make_shared<DBuf>(ext_words, c.stream));
     ext = keep.back()->p;
   }
-  const uint32_t* run_src = nullptr;  // a copy in the making: adjacent host columns
-  uint32_t* run_dst = nullptr;
-  size_t run_words = 0;
-  auto flush = [&] {
-    if (run_words) LG_CK(cudaMemcpyAsync(run_dst, run_src, run_words * 4, cudaMemcpyHostToDevice, c.stream));
-    run_words = 0;
-  };
+  HostCopies copies(c.stream);
   auto device = [&](const uint32_t* col, size_t n) -> const uint32_t* {
     if (on_device) return col;
     uint32_t* dst = up;
     up += n;
-    if (run_words && col == run_src + run_words) {
-      run_words += n;
-    } else {
-      flush();
-      run_src = col;
-      run_dst = dst;
-      run_words = n;
-    }
+    copies.add(col, dst, n);
     return dst;
   };
   std::vector<GroupSpec> gs;
@@ -391,7 +378,7 @@ std::vector<GroupSpec> batch_groups(Ctx& c, uint32_t n_groups, const uint64_t* r
     }
     gs.push_back(s);
   }
-  flush();
+  copies.flush();
   for (size_t first = 0; first < ext_cols.size(); first += 65535) {  // grid y: at most 65535 columns a launch
     const size_t cnt = std::min<size_t>(65535, ext_cols.size() - first);
     keep.push_back(upload_vec(c, std::vector<RowsCol>(ext_cols.begin() + first, ext_cols.begin() + first + cnt)));

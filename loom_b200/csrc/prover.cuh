@@ -465,8 +465,7 @@ struct Prover {
   // `split` (lg_prove, tuning upload_split), the columns round 0 commits go
   // up first on the main stream and the others on the side stream right
   // after them, while round 0 runs (await_upload joins them); otherwise
-  // every column goes up on the main stream.  Copies of columns that follow
-  // one another in host and device memory merge.
+  // every column goes up on the main stream (HostCopies).
   void setup(const uint32_t* const* witness, bool on_device, bool split = false) {
     init_order();
     size_t total_words = 0;
@@ -526,21 +525,12 @@ struct Prover {
         if (!any_late) std::fill(early.begin(), early.end(), 1);
       }
       auto copy = [&](bool want, cudaStream_t s) {
-        const uint32_t* run_src = nullptr;
-        uint32_t* run_dst = nullptr;
-        size_t run_words = 0;
-        auto flush = [&]() {
-          if (run_words) LG_CK(cudaMemcpyAsync(run_dst, run_src, run_words * 4, cudaMemcpyHostToDevice, s));
-          run_words = 0;
-        };
+        HostCopies up(s);
         for (uint32_t col = 0; col < pg.columns.size(); col++) {
           if (pg.columns[col].kind != KIND_WITNESS || (early[col] != 0) != want) continue;
-          const size_t n = mod_n(pg.columns[col].module);
-          uint32_t* dst = col_buf[col]->p;
-          if (run_words && src[col] == run_src + run_words && dst == run_dst + run_words) run_words += n;
-          else { flush(); run_src = src[col]; run_dst = dst; run_words = n; }
+          up.add(src[col], col_buf[col]->p, mod_n(pg.columns[col].module));
         }
-        flush();
+        up.flush();
       };
       copy(true, c.stream);
       if (any_late) {
