@@ -695,6 +695,7 @@ int lg_rs_encode(lg_ctx* ctx, const uint32_t* in, uint64_t n_rows, uint32_t n_co
     if (!in || !out || n_rows < 2 || (n_rows & (n_rows - 1))) throw Error(LG_ERR_INVALID, "bad arguments");
     uint32_t logn = 0;
     while ((1ull << logn) < n_rows) logn++;
+    check_ntt_size((int)logn);
     // device columns are encoded in place of staged copies, unless they overlap
     // or the output is not aligned to the transforms' 16-byte stores
     const size_t words = n_rows * n_cols;
