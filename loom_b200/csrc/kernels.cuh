@@ -600,7 +600,8 @@ __global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, con
   }
 }
 
-// Permutation test hook: one state of 24 words per group of six lanes.
+// Permutations of states of 24 words: one state per group of six lanes, and
+// one per thread for as many states as occupy the GPU so (p2_per_thread).
 __global__ void k_p2_permute(uint32_t* states, uint64_t n) {
   __shared__ __align__(16) uint32_t keys[p2c_smem_words(4)];
   p2_load_full_keys(keys);
@@ -615,6 +616,16 @@ __global__ void k_p2_permute(uint32_t* states, uint64_t n) {
   p2c_permute(x, L, keys);
   if (active)
     for (int q = 0; q < 4; q++) states[i * 24 + 4 * L.idx + q] = x[q];
+}
+__global__ void __launch_bounds__(P2_MAX_BLOCK, 2) k_p2_permute1(uint32_t* states, uint64_t n) {
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  uint32_t s[24];
+#pragma unroll
+  for (int q = 0; q < 24; q++) s[q] = states[i * 24 + q];
+  p2_permute(s);
+#pragma unroll
+  for (int q = 0; q < 24; q++) states[i * 24 + q] = s[q];
 }
 
 // ---------------------------------------------------------------- expressions
