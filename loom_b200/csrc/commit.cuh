@@ -332,7 +332,7 @@ struct TreeDev {
 // sized for the widest level of a block.
 inline unsigned tail_threads(uint32_t top, int fold_first) {
   uint32_t perms = std::max(1u, fold_first ? top : top / 2);
-  return std::min(1024u, (perms + 4) / 5 * 32);
+  return std::min((uint32_t)MERKLE_TAIL_BLOCK, (perms + 4) / 5 * 32);
 }
 
 // nodes must already hold the leaves at [n_leaves, 2 n_leaves).  Reads the
