@@ -31,9 +31,10 @@ from . import field as F
 CANDIDATES: Dict[str, Sequence[int]] = {
     "lde_split": (0, 1),
     "lde_fwd_threads": (256, 512, 1024),
-    "p2_leaf_min_per_sm": (32, 64, 128, 256, 512),
-    "p2_inject_min_per_sm": (64, 128, 256, 512, 1 << 20),
-    "p2_node_min_per_sm": (128, 256, 512, 1024, 2048),
+    # on both sides of the line where the two lane mappings meet
+    "p2_leaf_min_per_sm": (14, 20, 28, 40, 64, 128),
+    "p2_inject_min_per_sm": (14, 20, 28, 40, 64, 128, 1 << 20),
+    "p2_node_min_per_sm": (14, 20, 28, 40, 64, 128),
     "merkle_tail": (16, 32, 64, 128),
     "merkle_subtree": (0, 8, 16, 32, 64),
     "inject_block": (32, 64, 128),
