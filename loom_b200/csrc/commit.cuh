@@ -148,12 +148,11 @@ inline void big_fwd(Ctx& c, const FwdPlan& plan, const char* tag, double bytes_p
   });
 }
 
-inline BigNtt big_job(const uint32_t* in, uint32_t* out, uint32_t c0, bool bitrev_out) {
+inline BigNtt big_job(const uint32_t* in, uint32_t* out, uint32_t c0) {
   BigNtt j{};
   j.in = in;
   j.out = out;
   j.c0 = c0;
-  j.out_bitrev = bitrev_out ? 1 : 0;
   return j;
 }
 
@@ -178,7 +177,7 @@ inline void launch_lde(Ctx& c, const std::vector<LdeLane>& lanes, uint32_t log_n
           LG_CK(cudaMemcpyAsync(lanes[i].coef, lanes[i].src, n * 4, cudaMemcpyDeviceToDevice, c.stream));
       } else {
         uint32_t* dst = lanes[i].coef ? lanes[i].coef : tmp->p + i * n;
-        inv_jobs.push_back(big_job(lanes[i].src, dst, inv(to_mont((uint32_t)n)), false));
+        inv_jobs.push_back(big_job(lanes[i].src, dst, inv(to_mont((uint32_t)n))));
         inv_jobs.back().coset0 = lanes[i].out;       // <w_n> itself: the values in bit-reversed order
         inv_jobs.back().scratch = lanes[i].out + n;  // coset 1, not written before the forward transforms
         coef[i] = dst;

@@ -6,9 +6,8 @@
 // Pass A: for a tile of 16 consecutive k1, the length-C transforms over k2
 // (the tile's 16 columns are read 64 bytes at a time), times w_n^(j2 k1), into
 // scratch[j2 R + k1].  Pass B: for a tile of 16 consecutive j2, the length-R
-// transforms over k1 (scratch rows, contiguous), stored in natural order
-// (X[j]) or in bit-reversed order (out[bitrev(j)], what reedsolomon.Encode
-// produces).  Input scaling x[k] * c0 * t1[k] * t2[(e k) mod m2] covers 1/n
+// transforms over k1 (scratch rows, contiguous), stored in natural order.
+// Input scaling x[k] * c0 * t1[k] * t2[(e k) mod m2] covers 1/n
 // and the coset shifts.
 //
 // The 16 sub-transforms of a tile run together in shared memory with the
@@ -33,7 +32,6 @@ struct BigNtt {
   uint32_t m2_mask, e2;    // t2 index = (e2 * k) & m2_mask
   uint32_t c0;             // constant factor (Montgomery)
   uint32_t c0c, c0s;       // c0 canonical and its Shoup companion (big_ntt sets them)
-  int out_bitrev;
   uint32_t* coset0;        // pass A also writes its input in bit-reversed order here (16-byte aligned; null: no)
 };
 
@@ -49,19 +47,15 @@ __host__ __device__ constexpr size_t tile_words(int logl) {
 // tables of 2^LOGL points).  Pass 0 takes its
 // inputs from first(col, row) (global memory, or the staged tile), every pass
 // but the last writes back to S, the last hands each element to
-// store(col, row, value) — or, with STORE16 (DIF only: the last pass's local
-// bits are the lowest four), a thread's 16 consecutive rows 16 t .. 16 t + 15
-// of one column at once to store(col, t, v).  DIF: natural rows in,
-// bit-reversed rows out.
+// store(col, row, value).  DIF: natural rows in, bit-reversed rows out.
 struct NoTileHook {
   __device__ void operator()(uint32_t, uint32_t, int, uint32_t*) const {}
 };
 // `loaded(col, t, lo, v)` sees a thread's 16 inputs of pass 0 before its
 // butterflies and may change them.
-template <bool DIF, int LOGL, bool STORE16 = false, class First, class Store, class Loaded = NoTileHook>
+template <bool DIF, int LOGL, class First, class Store, class Loaded = NoTileHook>
 __device__ __forceinline__ void ntt16_tile(uint32_t* S, const uint32_t* tw, bool inverse, First first, Store store,
                                            Loaded loaded = Loaded()) {
-  static_assert(!STORE16 || DIF, "16-row stores follow the DIF pass plan");
   constexpr uint32_t groups = (1u << LOGL) >> 4;  // per column
   constexpr int np = (LOGL - ((LOGL & 3) ? (LOGL & 3) : 4)) / 4 + 1;
   constexpr uint32_t comp = tw16_words(LOGL);
@@ -80,22 +74,11 @@ __device__ __forceinline__ void ntt16_tile(uint32_t* S, const uint32_t* tw, bool
       }
       if (p == 0) loaded(col, t, lo, v);
       pass16<DIF>(v, t, lo, s_lo, s_hi, ptab, comp, inverse);
-      if constexpr (STORE16) {
-        if (p == np - 1) {
-          store(col, t, v);
-          continue;
-        }
-      }
 #pragma unroll
       for (uint32_t r = 0; r < 16; r++) {
         const uint32_t row = grp_index(t, r, lo);
-        if constexpr (!STORE16) {
-          if (p == np - 1) {
-            store(col, row, v[r]);
-            continue;
-          }
-        }
-        S[tile_addr(row, col)] = v[r];
+        if (p == np - 1) store(col, row, v[r]);
+        else S[tile_addr(row, col)] = v[r];
       }
     }
     __syncthreads();
@@ -168,24 +151,10 @@ __global__ void __launch_bounds__(512, 2) k_big_pass_b(const BigNtt* jobs, int l
   cp_async_wait_all();
   __syncthreads();
   auto first = [&](uint32_t col, uint32_t k1) { return S[tile_addr(k1, col)]; };
-  if (J.out_bitrev) {
-    // out[bitrev_C(j2) R + q] = X[C bitrev_R(q) + j2]: position q holds
-    // j1 = bitrev_R(q); a thread's rows q = 16 t .. 16 t + 15 are 64
-    // contiguous bytes of one output row
-    auto store = [&](uint32_t col, uint32_t t, const uint32_t* v) {
-      uint4* o = reinterpret_cast<uint4*>(J.out + (uint64_t)bitrev32(j2_0 + col, logc) * R + 16 * t);
-      o[0] = make_uint4(v[0], v[1], v[2], v[3]);
-      o[1] = make_uint4(v[4], v[5], v[6], v[7]);
-      o[2] = make_uint4(v[8], v[9], v[10], v[11]);
-      o[3] = make_uint4(v[12], v[13], v[14], v[15]);
-    };
-    ntt16_tile<true, LOGR, true>(S, tw_r, inverse != 0, first, store);
-  } else {
-    auto store = [&](uint32_t col, uint32_t q, uint32_t v) {
-      J.out[(uint64_t)C * bitrev32(q, LOGR) + j2_0 + col] = v;
-    };
-    ntt16_tile<true, LOGR>(S, tw_r, inverse != 0, first, store);
-  }
+  auto store = [&](uint32_t col, uint32_t q, uint32_t v) {
+    J.out[(uint64_t)C * bitrev32(q, LOGR) + j2_0 + col] = v;
+  };
+  ntt16_tile<true, LOGR>(S, tw_r, inverse != 0, first, store);
 }
 
 // ---------------------------------------------------------------- forward tree

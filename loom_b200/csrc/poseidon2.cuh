@@ -18,17 +18,14 @@ static const uint32_t P2_DIAG_H[24] = LG_P2_DIAG_INIT;
 #ifdef __CUDACC__
 __constant__ uint32_t P2_FULL_RK_D[6][24] = LG_P2_FULL_RK_INIT;
 __constant__ uint32_t P2_PARTIAL_RK_D[21] = LG_P2_PARTIAL_RK_INIT;
-__constant__ uint32_t P2_DIAG_D[24] = LG_P2_DIAG_INIT;
 #endif
 
 #ifdef __CUDA_ARCH__
 #define LG_P2_FULL_RK P2_FULL_RK_D
 #define LG_P2_PARTIAL_RK P2_PARTIAL_RK_D
-#define LG_P2_DIAG P2_DIAG_D
 #else
 #define LG_P2_FULL_RK P2_FULL_RK_H
 #define LG_P2_PARTIAL_RK P2_PARTIAL_RK_H
-#define LG_P2_DIAG P2_DIAG_H
 #endif
 
 LG_HD void p2_m4(uint32_t& x0, uint32_t& x1, uint32_t& x2, uint32_t& x3) {
@@ -58,20 +55,6 @@ LG_HD void p2_external(uint32_t s[24]) {
   }
 }
 
-LG_HD void p2_internal(uint32_t s[24]) {
-  // pairwise sum: 5 dependent additions instead of 23
-  uint32_t t[12];
-#pragma unroll
-  for (int i = 0; i < 12; i++) t[i] = add(s[2 * i], s[2 * i + 1]);
-#pragma unroll
-  for (int i = 0; i < 6; i++) t[i] = add(t[2 * i], t[2 * i + 1]);
-#pragma unroll
-  for (int i = 0; i < 3; i++) t[i] = add(t[2 * i], t[2 * i + 1]);
-  const uint32_t sum = add(add(t[0], t[1]), t[2]);
-#pragma unroll
-  for (int i = 0; i < 24; i++) s[i] = add(sum, mul(s[i], LG_P2_DIAG[i]));
-}
-
 LG_HD uint32_t p2_cube(uint32_t x) { return mul(mul_lazy(x, x), x); }
 
 // The round loops stay rolled: a fully unrolled permutation is more code than
@@ -95,7 +78,7 @@ constexpr uint32_t P2_DIAG_C[24] = LG_P2_DIAG_INIT;
 static_assert(P2_DIAG_C[1] == MONT_ONE, "internal diagonal entry 1 is 1");
 
 // The internal diagonal as canonical constants with their Shoup companions
-// (products by d_i need no 64-bit multiply), and 23 for the carried sum.
+// (products by d_i need no 64-bit multiply).
 struct P2DiagShoup { uint32_t w[24], ws[24]; };
 constexpr P2DiagShoup make_p2_diag_shoup() {
   P2DiagShoup d{};
@@ -108,14 +91,6 @@ constexpr P2DiagShoup make_p2_diag_shoup() {
 constexpr P2DiagShoup P2_DSH_H = make_p2_diag_shoup();
 static_assert(P2_DSH_H.w[1] == 1, "internal diagonal entry 1 is 1");
 static_assert(P2_DSH_H.w[0] == P - 2, "internal diagonal entry 0 is -2: s_0 <- sum + d_0 u = R - u");
-#ifdef __CUDACC__
-__constant__ P2DiagShoup P2_DSH_D = make_p2_diag_shoup();
-#endif
-#ifdef __CUDA_ARCH__
-#define LG_P2_DSH P2_DSH_D
-#else
-#define LG_P2_DSH P2_DSH_H
-#endif
 constexpr uint32_t C23 = 23, C23_SH = shoup(23);  // the carried sum (p2_coop.cuh)
 
 // Products by +-2^-k (17 of the 24 diagonal entries, and squares of them).  With

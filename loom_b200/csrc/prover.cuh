@@ -1247,7 +1247,7 @@ struct Prover {
       const size_t n = (size_t)1 << logn;
       if ((int)logn > SMEM_NTT_MAX_LOG) {
         std::vector<BigNtt> jobs;
-        for (uint32_t* l : lanes) jobs.push_back(big_job(l, l, inv(to_mont((uint32_t)n)), false));
+        for (uint32_t* l : lanes) jobs.push_back(big_job(l, l, inv(to_mont((uint32_t)n))));
         big_ntt(c, jobs, (int)logn, true, "quotient_intt", 8.0 * n);
         return;
       }
@@ -1289,7 +1289,7 @@ struct Prover {
           const uint32_t* gp = c.gpowers((int)logn, false);
           for (auto& L : kv.second)
             for (int cc = 0; cc < 4; cc++) {
-              BigNtt j = big_job(L.src, L.out + (size_t)cc * n, MONT_ONE, false);
+              BigNtt j = big_job(L.src, L.out + (size_t)cc * n, MONT_ONE);
               j.t1 = gp;
               j.t2 = tw4;
               j.m2_mask = (uint32_t)((n << RATE_LOG) - 1);
@@ -1368,7 +1368,7 @@ struct Prover {
         size_t n = (size_t)1 << kv.first;
         if ((int)kv.first > SMEM_NTT_MAX_LOG) {
           std::vector<BigNtt> jobs;
-          for (uint32_t* l : kv.second) jobs.push_back(big_job(l, l, inv(to_mont((uint32_t)n)), false));
+          for (uint32_t* l : kv.second) jobs.push_back(big_job(l, l, inv(to_mont((uint32_t)n))));
           big_ntt(c, jobs, (int)kv.first, true, "quotient_intt", 8.0 * n);
           continue;
         }
