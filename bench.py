@@ -645,9 +645,13 @@ def main():
                     "traffic": traffic_of(k, per), "algorithmic_bytes_per_launch": round(per),
                     "avg_launch_ms": round(v["ms"] / v["launches"], 5), "share": shares[k]}
 
-        # Poseidon2 kernels: integer-multiply bound; 165 cubes and 14 diagonal
-        # products in each of 21 partial rounds, 3 IMAD per product = 1872 per
-        # width-24 permutation.
+        # Poseidon2 kernels: integer-multiply bound.  Multiplies that a width-24
+        # permutation issues in one thread (poseidon2.cuh): 144 cubes of the
+        # full rounds at 6; each of 21 partial rounds a cube (6), three Shoup
+        # products (3 each) and six shift products (1) for the pairs, three for
+        # the singles, two for the carried sum and its reduction = 26; 33 and 13
+        # on the way into and out of the pairs: 864 + 546 + 46 = 1456.  Beside
+        # it the rate at the fixed definition of 3336 IMAD a permutation.
         sm_count = torch.cuda.get_device_properties(device).multi_processor_count
         clk_mhz = clk.get("sm_mhz") or peaks.get("sm_max_mhz") or 1965.0
         imad_peak = sm_count * 64 * clk_mhz * 1e6
@@ -658,8 +662,9 @@ def main():
         if p2_ms:
             ach = p2_perms / (p2_ms * 1e-3)
             p2_roof = {"kernels": list(p2), "bound": "int32", "achieved": round(ach / 1e9, 3),
-                       "peak": round(imad_peak / 1872 / 1e9, 3), "unit": "Gperm/s",
-                       "frac": round(ach / (imad_peak / 1872), 4),
+                       "peak": round(imad_peak / 1456 / 1e9, 3), "unit": "Gperm/s",
+                       "frac": round(ach / (imad_peak / 1456), 4),
+                       "frac_at_3336_imad": round(ach / (imad_peak / 3336), 4),
                        "peak_source": f"nominal {sm_count} SMs x 64 IMAD/clk at the sampled {clk_mhz:.0f} MHz",
                        "share": round(p2_ms / total_k, 4)}
         hbm_dom = max((k for k in rep if k in hbm_kernels), key=lambda k: rep[k]["ms"], default=None)
