@@ -5,7 +5,9 @@
  * The Go prover binds these functions through a cgo shim package; Python
  * binds them through ctypes (loom_b200/_lib.py).  Signatures use plain pointers and
  * sizes only.  Every function returns an int status (LG_OK = 0) and never
- * aborts; lg_last_error() describes the last failure on a context.
+ * aborts; lg_last_error() describes the last failure on a context.  A call
+ * that fails (LG_ERR_BUFFER aside, which answers a size query) has ended all
+ * the device work that it had begun when it returns.
  *
  * Field data: KoalaBear (p = 2^31 - 2^24 + 1) elements are 32-bit
  * Montgomery words (R = 2^32), the in-memory layout of gnark-crypto's
@@ -98,7 +100,10 @@ typedef struct lg_session lg_session;
  * `device`.  `hbm_budget` caps the device bytes the context may hold at once
  * (0: no cap); an allocation past it fails with LG_ERR_OOM.  Replaces nothing
  * in the reference: the Go prover has no device state; the cgo shim creates
- * one context per GPU.  Release every handle made on a context before
+ * one context per GPU.  What a context keeps between calls counts too: its
+ * twiddle tables, of which the longest takes 16 bytes per row of the largest
+ * transform above 2^14 rows that it has run (4 MiB at 2^18, 64 MiB at 2^22
+ * rows), and its programs.  Release every handle made on a context before
  * destroying it. */
 int lg_ctx_create(int device, size_t hbm_budget, lg_ctx** out);
 void lg_ctx_destroy(lg_ctx* ctx);
@@ -303,7 +308,8 @@ void lg_release(void* handle);
 
 /* reedsolomon.Encoder.Encode (internal/reedsolomon/rs.go:52-70) on
  * `n_cols` base columns of n_rows rows stored one after another in `in`;
- * writes 4 * n_rows bit-reversed evaluations per column to `out`. */
+ * writes 4 * n_rows bit-reversed evaluations per column to `out`.  More than
+ * 2^22 rows: LG_ERR_UNSUPPORTED. */
 int lg_rs_encode(lg_ctx* ctx, const uint32_t* in, uint64_t n_rows, uint32_t n_cols, uint32_t* out, int on_device);
 
 /* poseidon2.Permutation (width 24) applied in place to n_states states of

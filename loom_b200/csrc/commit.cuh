@@ -262,12 +262,12 @@ inline void launch_lde(Ctx& c, const std::vector<LdeLane>& lanes, uint32_t log_n
 // Poseidon2 lane mapping for a launch of `parallel` independent permutation
 // chains (leaves, nodes of one level): with at least `per_sm` of them per SM,
 // one thread per chain (fewest instructions per permutation); otherwise six
-// lanes per chain for a dependent chain shorter by half.  The line lies where
-// the two take the same time: 28 chains per SM (B200, 148 SMs: 4144 chains).
-// Measured, six lanes against one thread: a tree of 2^13 leaves (the level of
-// 4096 nodes) 99 / 94 us, of 2^14 (8192) 120 / 109, of 2^15 145 / 119; eight
-// chained injections of width 4096 175 / 185 us, 8192 199 / 191, 16384
-// 268 / 214 (Ctx::tune).
+// lanes per chain for a dependent chain shorter by half.  The line, 28 chains
+// per SM (B200, 148 SMs: 4144 chains), lies between the last width at which six
+// lanes are faster and the first at which one thread is.  Measured for a
+// tree's widest level, six lanes / one thread: 4096 nodes (2^13 leaves) 90.1 /
+// 91.3 us, 8192 112.6 / 100.5, 16384 138 / 127; for eight injections into it:
+// 146 / 157, 173 / 165, 230 / 175 (Ctx::tune).
 inline bool p2_per_thread(const Ctx& c, uint64_t parallel, uint32_t per_sm) {
   return c.leaf_mapping == 1 || (c.leaf_mapping == 0 && parallel >= (uint64_t)c.sm_count * per_sm);
 }
@@ -364,8 +364,8 @@ inline bool build_tree(Ctx& c, TreeDev& t, bool read_root = true, const FsTail* 
     uint32_t cnt = (uint32_t)(next - first);
     c.timed("merkle_inject", 96.0 * start * cnt, (double)start * cnt, [&] {
       if (p2_per_thread(c, start, c.tune.p2_inject_min_per_sm)) {
-        // small blocks (one warp by default): chains are few (down to ~200
-        // per SM) and long, so small blocks spread them evenly over the SMs
+        // small blocks (one warp by default): chains are few (down to 28 per
+        // SM) and long, so small blocks spread them evenly over the SMs
         const unsigned ib = std::min<unsigned>(c.tune.inject_block, P2_MAX_BLOCK);
         k_merkle_inject1<<<(start + ib - 1) / ib, ib, 0, c.stream>>>(t.nodes->p, start, tab, cnt);
       } else

@@ -4,8 +4,8 @@
 //
 // E6 = E2[v]/(v^3 - (u + 1)), E2 = F[u]/(u^2 - 3) (recursion/e6.go:21-53),
 // coefficient order [B0.A0, B0.A1, B1.A0, B1.A1, B2.A0, B2.A1]
-// (internal/hash/hash.go:59-68).  Products use Karatsuba at both levels
-// (3 base products per E2 product, 6 E2 products per E6 product).
+// (internal/hash/hash.go:59-68).  Products are schoolbook sums with one
+// reduction per coefficient (e2_mul, e6_mul).
 //
 // Every function is __host__ __device__: the host-side Fiat-Shamir transcript
 // uses the same code as the kernels.

@@ -1331,8 +1331,8 @@ template <int ROWS> __device__ __forceinline__ void deep_inverses(const E6& z, c
 // coefficients are staged in shared memory.  ROWMAJOR: rows of six words out,
 // one point, the denominators computed here.  NP: points held in registers
 // (at least the job's).
-// What bounds it: the integer-multiply pipe (6 wide products per lane and row).
-// 48 lanes of 2^20 rows on B200: 128 us a call (349 us lane by lane, with the
+// What bounds it: the integer-multiply pipe (6 wide products per lane and row;
+// 77% of its peak, DRAM 27%).  48 lanes of 2^20 rows on B200: 128 us a call (349 us lane by lane, with the
 // points' sums in local memory and a transposing pass after it).
 constexpr int DEEP_BLOCK = 128, DEEP_STAGE = 64;
 template <int NP, int ROWS, bool ROWMAJOR>
@@ -1612,8 +1612,9 @@ __global__ void k_fold(const uint32_t* layer, uint64_t n, const uint32_t* alpha_
 // tables that stay in L1 (mul_split, ntt_large.cuh: w_n^-e = w_n^(n - e))
 // rather than a scattered read of a table as long as the layer.  VEC: 16- and
 // 8-byte accesses (the caller's rows aligned to 16 bytes).
-// What bounds it: HBM and the integer pipes about equally (72 B and 30
-// products per output row).  2^22 rows on B200: 48 us a call, 0.48 of the
+// What bounds it: the multiply pipe, then HBM (an extension product and twelve
+// Shoup products for 72 B per output row: 71% and 45% of their peaks).  2^22
+// rows on B200: 48 us a call, 0.48 of the
 // measured HBM rate (257 us with a copy in, a transpose, the fold, a transpose
 // back and a copy out).
 constexpr int FOLD_SPLIT = 11;

@@ -171,11 +171,14 @@ __global__ void __launch_bounds__(512, 2) k_big_pass_b(const BigNtt* jobs, int l
 // place in the output.  One table of tau (with Shoup companions) serves every
 // size and coset.
 //
-// What bounds it: the integer pipes (eight instructions a butterfly).  Per
-// element of a 2^18-point transform the four-step form took 118 + 75
-// instructions.  Rate-4 encoding of 128 columns of 2^18 rows on B200: 978 us,
-// 1478 us with four-step coset transforms (a fourth of them for coset 0,
-// which pass A of the inverse transform now writes as it reads the values).
+// What bounds it: pass A the integer pipes (eight instructions a butterfly:
+// multiply 58%, ALU 61%, issue 63% of their peaks), pass B the L1 data pipe
+// (76%: the words' passes through shared memory and 120 B of twiddles per 16
+// words of one column).  Per element of a 2^18-point transform the four-step
+// form took 118 + 75 instructions, the tree 73 + 47.  Rate-4 encoding of 128
+// columns of 2^18 rows on B200: 976 us, 1478 us with four-step coset transforms
+// (a fourth of them for coset 0, which pass A of the inverse transform now
+// writes as it reads the values).
 struct FwdJob { const uint32_t* in; uint32_t* out; uint32_t node; };  // node: the coset a
 
 // The first `levels` levels under node N on 16 registers (a group's elements,

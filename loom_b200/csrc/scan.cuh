@@ -96,8 +96,9 @@ inline uint32_t gp_tile(uint64_t n) { return n <= 1u << 16 ? GP_TILE_S : n <= 1u
 // for all R rows and three E6 products a row, where an inversion takes about
 // six.  The denominators are taken from the back and the numerators from the
 // front, one row at a time, so only the products stay in registers.
-// What bounds it: the integer-multiply pipe (about five E6 products a row)
-// and, for few tiles, the dependent products of the scan and the inversion.
+// What bounds it: the integer-multiply pipe (about five E6 products a row; 61%
+// of its peak) and, with 16 warps an SM, the loads' latency (long scoreboard 2.2
+// per issue; a row's 24 B are fetched where they lie, L1 at 47%); for few tiles, the dependent products of the scan and the inversion.
 // 512 threads an SM, 128 registers each: with both operands of every row held
 // (210 registers) 1,000,003 rows took 162 us and not 127 (start to end; 98 with
 // the extension products of one reduction per coefficient).
@@ -147,8 +148,8 @@ __global__ void __launch_bounds__(T, 512 / T) k_rows_scan(const uint32_t* num, c
 
 // x[i] *= the product of the tiles before tile i / tile.  PREFIX: `pre` holds
 // those products; otherwise the totals, which every block multiplies up to its
-// own tile (at most a few E6 products a thread: n / tile^2 and the block's
-// reduction), saving the launch between.
+// own tile (the tiles before it over T threads, at most four E6 products each,
+// and the block's reduction), saving the launch between.
 // The block's rows are loaded before that, so the two overlap.
 template <int T, int R, bool VEC, bool PREFIX>
 __global__ void __launch_bounds__(T, 512 / T) k_rows_apply(uint32_t* x, uint64_t n, const uint32_t* pre) {
