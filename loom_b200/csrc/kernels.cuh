@@ -544,12 +544,15 @@ __global__ void __launch_bounds__(P2_MAX_BLOCK, 2) k_merkle_inject1(uint32_t* no
 // as k_fs_challenge, which it replaces for the FRI layer trees.
 struct InjRef { const uint32_t* leaves; uint32_t width; };
 struct FsTail { const uint32_t* pre; uint32_t n_pre; const uint32_t* prev; uint32_t* out; };
-// A block of 1024 threads leaves each 64 registers, which is just what the
+// A block of 1024 threads would leave each 64 registers, which is just what the
 // kernel takes (71 when nvcc compiles the unit in parts, and such a block does
-// not start); 512 are declared, and the widest levels take more turns.
+// not start); blocks have at most 512, with room for twice as many, and the
+// widest levels take more turns.  Not a launch bound: compiled for one, the
+// kernel has the same registers and is 1-4 us slower a tree of 2^11 or 2^13
+// leaves (B200: 84 -> 88 and 96 -> 97 us).
 constexpr int MERKLE_TAIL_BLOCK = 512;
-__global__ void __launch_bounds__(MERKLE_TAIL_BLOCK) k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first,
-                                                                   const InjRef* inj, uint32_t n_inj, FsTail fs) {
+__global__ void k_merkle_tail(uint32_t* nodes, uint32_t top, int fold_first, const InjRef* inj, uint32_t n_inj,
+                              FsTail fs) {
   extern __shared__ __align__(16) uint32_t keys[];  // p2c_smem_words(warps)
   __shared__ const uint32_t* chain[64];
   __shared__ uint32_t msg[64];
